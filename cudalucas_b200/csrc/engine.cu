@@ -79,16 +79,12 @@ struct TallArgs {
   int pf;  // > 0: prefetch into L2 the column pair pf units ahead (state larger than L2)
 };
 
-// Ready flags per wide-pass CTA: the specialised kernels hand the carry over
-// warp by warp (at most 32 warps per CTA); the generic ones use the first.
-constexpr int kWarpFlags = 32;
-
 struct WideArgs {
   double2 *A;
   const double2 *stw;   // stage twiddles of the specialised row transform
   int32_t *xint;
-  long long *carry;     // packed carries, one row of W per CTA
-  uint32_t *flags;      // ready flags: kWarpFlags per CTA (one per warp)
+  long long *carry;     // carries, one row of W per CTA: packed pairs (generic) or doubles
+  uint32_t *flags;      // ready flags of the generic kernels, one per CTA
   const double2 *twW;
   const int32_t *rowE;  // ((-(2*m2+t)*b) mod n), 2H entries
   const double *rowW;   // 2^(rowE/n)
@@ -101,11 +97,14 @@ struct WideArgs {
   int W, H, G, ngroups;
   int pf;  // > 0: prefetch into L2 the row group pf tickets ahead (state larger than L2)
   uint32_t q, n, b, qn;
-  // specialised kernels: column m1 = t + r*TR has exponent colF[t] - colD[r]
-  // (mod n), i.e. weight colW[t] * colS[r] (times 2 when it wraps)
-  int colD[16];
+  double inv_q, inv_n, inv_H;  // reciprocals for udiv_est
+  // specialised kernels: column m1 = t + r*TR has exponent colF[t] - D_r
+  // (mod n), i.e. weight colW[t] * colS[r] (times 2 when it wraps); exponents
+  // as fractions of a turn (see WordSize): D_r in colD, b in lim
+  double turn;  // 2^32 / n
+  uint32_t lim;
+  uint32_t colD[16];
   double colS[16], colSi[16];
-  double colS2[16], colSi2[16];  // 2*colS, 0.5*colSi (wrapped exponents)
 };
 
 __device__ __forceinline__ double2 omegaN(const double2 *__restrict__ thi, const double2 *__restrict__ tlo,
@@ -1023,6 +1022,25 @@ static void free_ctx(ll_ctx *c) {
   delete c;
 }
 
+// The row pass's constants that follow from q, n, H and the row kernel.
+static void fill_wide_constants(WideArgs &wa, const Shape &s) {
+  const uint32_t n = wa.n;
+  wa.inv_q = 1.0 / (double)wa.q;
+  wa.inv_n = 1.0 / (double)n;
+  wa.inv_H = 1.0 / (double)s.H;
+  if (!s.sw) return;
+  wa.turn = 4294967296.0 / (double)n;
+  wa.lim = (uint32_t)((double)wa.b * wa.turn);
+  const long long TR = s.sw->tr;
+  for (int r = 0; r < 16; ++r) {
+    // column m1 = t + r*TR: exponent colF[t] - D (mod n), D = r*TR*2H*b mod n
+    const long long D = (long long)((unsigned __int128)r * TR * 2 * s.H % n * wa.b % n);
+    wa.colD[r] = (uint32_t)((double)D * wa.turn);
+    wa.colS[r] = (double)exp2l(-(long double)D / (long double)n);
+    wa.colSi[r] = (double)exp2l((long double)D / (long double)n);
+  }
+}
+
 static ll_status build_tables(ll_ctx *ctx) {
   const int W = ctx->shape.W, H = ctx->shape.H, N = ctx->N;
   const uint32_t n = ctx->n, b = ctx->b;
@@ -1126,12 +1144,13 @@ ll_status ll_create(int device, uint32_t q, uint32_t n, const ll_tuning *tuning,
     if ((e = cudaMalloc((void **)&ctx->A, sizeof(double2) * (size_t)ctx->N)) != cudaSuccess ||
         (e = cudaMalloc((void **)&ctx->xint, sizeof(int32_t) * (size_t)n)) != cudaSuccess ||
         (e = cudaMalloc((void **)&ctx->carry, sizeof(long long) * (size_t)ngroups * s.W)) != cudaSuccess ||
-        (e = cudaMalloc((void **)&ctx->flags, sizeof(uint32_t) * kWarpFlags * (size_t)ngroups)) != cudaSuccess ||
+        (e = cudaMalloc((void **)&ctx->flags, sizeof(uint32_t) * (size_t)ngroups)) != cudaSuccess ||
         (e = cudaMalloc((void **)&ctx->st, sizeof(DevState))) != cudaSuccess) {
       rc = e == cudaErrorMemoryAllocation ? LL_ERR_NOMEM : cuda_fail(ctx, e, "cudaMalloc");
       break;
     }
-    if ((e = cudaMemset(ctx->flags, 0, sizeof(uint32_t) * kWarpFlags * (size_t)ngroups)) != cudaSuccess ||
+    if ((e = cudaMemset(ctx->flags, 0, sizeof(uint32_t) * (size_t)ngroups)) != cudaSuccess ||
+        (s.sw && (e = cudaMemset(ctx->carry, kNoCarryByte, sizeof(long long) * (size_t)ngroups * s.W)) != cudaSuccess) ||
         (e = cudaMemset(ctx->st, 0, sizeof(DevState))) != cudaSuccess) {
       rc = cuda_fail(ctx, e, "cudaMemset");
       break;
@@ -1277,18 +1296,7 @@ ll_status ll_create(int device, uint32_t q, uint32_t n, const ll_tuning *tuning,
         if (s.st->ppc == 1 && s.H >= 2048) ta.pf = sms * bt;
       }
     }
-    if (s.sw) {
-      // column m1 = t + r*TR: exponent colF[t] - D_r (mod n), D_r = r*TR*2H*b mod n
-      const long long TR = s.sw->tr;
-      for (int r = 0; r < 16; ++r) {
-        const long long D = (long long)((unsigned __int128)r * TR * 2 * s.H % n * ctx->b % n);
-        wa.colD[r] = (int)D;
-        wa.colS[r] = (double)exp2l(-(long double)D / (long double)n);
-        wa.colSi[r] = (double)exp2l((long double)D / (long double)n);
-        wa.colS2[r] = 2.0 * wa.colS[r];
-        wa.colSi2[r] = 0.5 * wa.colSi[r];
-      }
-    }
+    fill_wide_constants(wa, s);
   } while (0);
   cudaSetDevice(prev);
   if (rc != LL_OK) {
@@ -1557,7 +1565,7 @@ uint64_t ll_context_bytes(uint32_t q, uint32_t n, const ll_tuning *tuning) {
   const uint64_t N = n / 2, W = (uint64_t)s.W, H = (uint64_t)s.H, ng = (uint64_t)(s.H / s.G);
   int ts = 0;
   while ((1 << (ts + 1)) * (long long)(1 << (ts + 1)) <= (long long)N * 4 && ts < 14) ++ts;
-  uint64_t b = 16 * N + 4ull * n + 8 * ng * W + 4 * kWarpFlags * ng + sizeof(DevState);  // state, digits, carries
+  uint64_t b = 16 * N + 4ull * n + 8 * ng * W + 4 * ng + sizeof(DevState);  // state, digits, carries
   b += 16 * (W + H) + 16 * (((uint64_t)1 << ts) + (N >> ts) + 1);                     // twiddles
   b += 20 * 2 * H + 20 * W;                                                           // weights
   if (s.sw) b += 16 * (uint64_t)s.sw->extra;
@@ -1838,7 +1846,7 @@ extern "C" ll_status ll_step_static(int device, uint32_t q, uint32_t n, uint32_t
   };
   double2 *A = (double2 *)dput(sizeof(double2) * (size_t)N);
   long long *carry = (long long *)dput(sizeof(long long) * (size_t)ngroups * W);
-  uint32_t *flags = (uint32_t *)dput(sizeof(uint32_t) * kWarpFlags * (size_t)ngroups);
+  uint32_t *flags = (uint32_t *)dput(sizeof(uint32_t) * (size_t)ngroups);
   DevState *dst = (DevState *)dput(sizeof(DevState));
   unsigned char *dtab = dput(table_bytes);
   if (o > kScratchBytes) return LL_ERR_ARG;  // shape needs more scratch than the static array holds
@@ -1874,23 +1882,14 @@ extern "C" ll_status ll_step_static(int device, uint32_t q, uint32_t n, uint32_t
   wa.colF = (const int32_t *)dev(h_cF); wa.colW = (const double *)dev(h_cW); wa.colWi = (const double *)dev(h_cWi);
   wa.st = dst; wa.pw = pw; wa.W = W; wa.H = H; wa.G = s.G; wa.ngroups = ngroups;
   wa.q = q; wa.n = n; wa.b = b; wa.qn = qn;
-  if (s.sw) {
-    const long long TR = s.sw->tr;
-    for (int r = 0; r < 16; ++r) {
-      const long long D = (long long)((unsigned __int128)r * TR * 2 * H % n * b % n);
-      wa.colD[r] = (int)D;
-      wa.colS[r] = (double)exp2l(-(long double)D / (long double)n);
-      wa.colSi[r] = (double)exp2l((long double)D / (long double)n);
-      wa.colS2[r] = 2.0 * wa.colS[r];
-      wa.colSi2[r] = 0.5 * wa.colSi[r];
-    }
-  }
+  fill_wide_constants(wa, s);
 
   // ---- state that must start at zero: flags, ticket, error, fault
   DevState hs{};
   hs.offset = offset;
   restore.enqueued = true;
-  if ((e = cudaMemsetAsync(flags, 0, sizeof(uint32_t) * kWarpFlags * (size_t)ngroups, st)) != cudaSuccess ||
+  if ((e = cudaMemsetAsync(flags, 0, sizeof(uint32_t) * (size_t)ngroups, st)) != cudaSuccess ||
+      (s.sw && (e = cudaMemsetAsync(carry, kNoCarryByte, sizeof(long long) * (size_t)ngroups * W, st)) != cudaSuccess) ||
       (e = cudaMemcpyAsync(dst, &hs, sizeof(DevState), cudaMemcpyHostToDevice, st)) != cudaSuccess ||
       (e = cudaMemcpyAsync(dtab, g_host_tables, table_bytes, cudaMemcpyHostToDevice, st)) != cudaSuccess)
     return LL_ERR_CUDA;

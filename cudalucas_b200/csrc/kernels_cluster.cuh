@@ -82,16 +82,6 @@ struct ClusterCfg {
                 "first and last row stages: one butterfly per thread, elements t + j*TWR");
 };
 
-// floor(x / d) for x < 2^58 and d < 2^31: an FP64 estimate (off by at most
-// one, its relative error is a few 2^-53 and the quotient is below 2^31),
-// then one exact correction step in integers.
-__device__ __forceinline__ uint32_t udiv_est(unsigned long long x, uint32_t d, double inv_d) {
-  unsigned long long e = (unsigned long long)((double)x * inv_d);
-  if (e * d > x) --e;
-  else if ((e + 1) * d <= x) ++e;
-  return (uint32_t)e;
-}
-
 // Point-to-point hand-off between two CTAs of the cluster through an
 // mbarrier in the receiver's shared memory: the sender's stores into the
 // receiver, a CTA barrier, then one release arrive on the receiver's
@@ -149,11 +139,12 @@ __global__ void __launch_bounds__(ClusterCfg<PR, TWR, PT, TC, C, RPC>::T, 1)
   using CF = ClusterCfg<PR, TWR, PT, TC, C, RPC>;
   constexpr int W = CF::W, H = CF::H, EPR = CF::EPR, PPC = CF::PPC, CS = CF::CS, RS = CF::RS, PS = CF::PS;
   constexpr int T = CF::T, TT = CF::TT, TW = CF::TW;
+  constexpr bool kIdleWarp = TT <= T - 32;
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ double2 sm[];
-  __shared__ float s_err[32];
-  __shared__ uint32_t s_fault;
+  __shared__ uint32_t s_sub[2];  // the element the -2 hits, and what its words lose
+  __shared__ double s_two[2];
   __shared__ __align__(8) uint64_t s_cbar;  // the previous CTA's carries have arrived
   const int rank = (int)cl.block_rank();
   const int tid = threadIdx.x;
@@ -161,19 +152,16 @@ __global__ void __launch_bounds__(ClusterCfg<PR, TWR, PT, TC, C, RPC>::T, 1)
   double2 *stw = sm + CF::o_stw, *stt = sm + CF::o_stt;
   double2 *cols = sm + CF::o_col, *ctw = sm + CF::o_ctw, *ptw = sm + CF::o_ptw;
   double2 *cwt = sm + CF::o_cwt;
-  int *cf = reinterpret_cast<int *>(sm + CF::o_cf);
+  uint32_t *cf = reinterpret_cast<uint32_t *>(sm + CF::o_cf);
   double *cin = reinterpret_cast<double *>(sm + CF::o_cin);
 
   // ---- set-up: tables, twiddles of the owned columns, the owned state
-  if (tid == 0) {
-    s_fault = 0;
-    mbar_init(&s_cbar, 1);  // one arrive per iteration: the previous CTA's
-  }
+  if (tid == 0) mbar_init(&s_cbar, 1);  // one arrive per iteration: the previous CTA's
   for (int i = tid; i < tw_size<PR>(); i += T) stw[i] = stwr[i];
   for (int i = tid; i < tw_size<PT>(); i += T) stt[i] = stwr[tw_size<PR>() + i];
   for (int i = tid; i < W; i += T) {
     cwt[i] = make_double2(wa.colW[i], wa.colWi[i]);
-    cf[i] = wa.colF[i];
+    cf[i] = (uint32_t)((double)wa.colF[i] * wa.turn);
   }
   for (int i = tid; i < 2 * PPC * H; i += T) {
     const int lc = i / H, m2 = i - lc * H;
@@ -194,29 +182,28 @@ __global__ void __launch_bounds__(ClusterCfg<PR, TWR, PT, TC, C, RPC>::T, 1)
   const bool wide = rank < CF::ROWCTAS && tid < TW;
   const int row = tid / TWR, t = tid - (tid / TWR) * TWR;
   const int m2 = rank * RPC + row;
-  const int n = (int)wa.n, bb = (int)wa.b, qn = (int)wa.qn;
-  const uint32_t q = wa.q, un = wa.n;
-  const double inv_q = 1.0 / (double)q, inv_n = 1.0 / (double)un;
-  int rE0 = 0, rE1 = 0;
+  const uint32_t q = wa.q;
+  // exponents as fractions of a turn (see WordSize): row plus column, which
+  // wrap by themselves
+  uint32_t rF0 = 0, rF1 = 0;
   double rW0 = 0.0, rW1 = 0.0, rWi0 = 0.0, rWi1 = 0.0;
   if (wide) {
-    rE0 = wa.rowE[2 * m2];
-    rE1 = wa.rowE[2 * m2 + 1];
+    rF0 = turn_fraction(wa.rowE[2 * m2], wa.turn);
+    rF1 = turn_fraction(wa.rowE[2 * m2 + 1], wa.turn);
     rW0 = wa.rowW[2 * m2];
     rW1 = wa.rowW[2 * m2 + 1];
     rWi0 = wa.rowWi[2 * m2];
     rWi1 = wa.rowWi[2 * m2 + 1];
   }
-  const double p2lo = (double)(1 << qn), p2hi = 2.0 * p2lo;
-  const double ip2lo = 1.0 / p2lo, ip2hi = 0.5 * ip2lo;
+  const WordSize ws(wa.lim, (int)wa.qn);
   // the carries of the last row go to the next CTA's carry row (into rank 0
   // shifted by one element)
   const bool wrap = rank == CF::ROWCTAS - 1;
   double *next_cin = cl.map_shared_rank(cin, (unsigned)(wrap ? 0 : rank + 1));
   const uint32_t next_cbar = mbar_remote(&s_cbar, (unsigned)(wrap ? 0 : rank + 1));
   uint32_t off = ta.st->offset;
-  double emax = 0.0;
-  bool out_of_range = false;
+  const uint32_t seen = ta.st->err_bits;
+  Readings rd;
   double2 *rw = rows + row * RS;
 
   // tall-pass thread: column `col` (local slot) of pair pl, thread tc of TC
@@ -236,6 +223,16 @@ __global__ void __launch_bounds__(ClusterCfg<PR, TWR, PT, TC, C, RPC>::T, 1)
   for (uint32_t it = 0; it < iters; ++it) {
     // CUDALucas.cu:1882: offset <- 2*offset mod q, once per iteration
     off = 2u * off >= q ? 2u * off - q : 2u * off;
+    // where the -2 falls: worked out by a warp that is idle in the column
+    // pass, if there is one (12K 4.65 -> 4.42 us per iteration), else by every
+    // row thread (by one busy warp for all: 8K 3.54 -> 3.61)
+    if (kIdleWarp && tid == T - 1) {
+      const MinusTwo two(off, wa);
+      s_sub[0] = two.m1;
+      s_sub[1] = two.m2;
+      s_two[0] = two.s0;
+      s_two[1] = two.s1;
+    }
     // ---------------------------------------------------------- tall pass
     if (tid < TT) {
       double2 *cc = cols + col * CS;
@@ -280,18 +277,22 @@ __global__ void __launch_bounds__(ClusterCfg<PR, TWR, PT, TC, C, RPC>::T, 1)
     cl.sync();  // every row buffer holds its row
     // ---------------------------------------------------------- wide pass
     if (wide) {
-      // the -2 (bit (offset+1) mod q, CUDALucas.cu:1882-1886): element
-      // j_sub, word w_sub of the thread that holds it
-      const uint32_t pos = off + 1 == q ? 0u : off + 1;
-      const uint32_t dw = udiv_est((unsigned long long)pos * un, q, inv_q);
-      const uint32_t sdw = udiv_est((unsigned long long)dw * q + un - 1, un, inv_n);
-      const double sub = (double)(1u << (pos - sdw));
-      int j_sub = -1;
-      {
-        const uint32_t me = dw >> 1, mm1 = me / (uint32_t)H, mm2 = me - mm1 * (uint32_t)H;
-        if ((int)mm2 == m2 && (int)(mm1 % TWR) == t) j_sub = (int)(mm1 / TWR);
+      // element register of this thread that the -2 hits, if any
+      uint32_t sub1, sub2;
+      double two0, two1;
+      if constexpr (kIdleWarp) {
+        sub1 = s_sub[0];
+        sub2 = s_sub[1];
+        two0 = s_two[0];
+        two1 = s_two[1];
+      } else {
+        const MinusTwo two(off, wa);
+        sub1 = two.m1;
+        sub2 = two.m2;
+        two0 = two.s0;
+        two1 = two.s1;
       }
-      const bool w_sub = dw & 1;
+      const int j_sub = (int)sub2 == m2 && (int)(sub1 % TWR) == t ? (int)(sub1 / TWR) : -1;
       // inverse row transform; its last stage leaves elements t + j*TWR in u[j]
       double2 u[EPR];
       auto ld = [&](int e, int, int) { return rw[pad(e)]; };
@@ -301,33 +302,23 @@ __global__ void __launch_bounds__(ClusterCfg<PR, TWR, PT, TC, C, RPC>::T, 1)
 #pragma unroll
       for (int j = 0; j < EPR; ++j) {
         const int m1 = t + j * TWR;
-        const int cfm = cf[m1];
+        const uint32_t cfm = cf[m1];
         const double cwi = cwt[m1].y;
-        int e0 = rE0 + cfm, e1 = rE1 + cfm;
-        const bool f0 = e0 >= n, f1 = e1 >= n;
-        if (f0) e0 -= n;
-        if (f1) e1 -= n;
-        const double t0 = u[j].x * (rWi0 * cwi * (f0 ? 2.0 : 1.0));
-        const double t1 = u[j].y * (rWi1 * cwi * (f1 ? 2.0 : 1.0));
-        double r0 = rint(t0), r1 = rint(t1);
-        emax = fmax(emax, fmax(fabs(t0 - r0), fabs(t1 - r1)));
-        // at 2^51 and above (or NaN) a double has no fraction bits left for
-        // the roundoff reading, and the exact carry split no longer holds
-        if (!(fabs(t0) < 0x1p51 && fabs(t1) < 0x1p51)) out_of_range = true;
+        const uint32_t f0 = rF0 + cfm, f1 = rF1 + cfm;
+        double P0, I0, P1, I1;
+        ws.at(f0, P0, I0);
+        ws.at(f1, P1, I1);
+        const double t0 = u[j].x * scale_exp(rWi0 * cwi, f0 < cfm ? kExpOne : 0);
+        const double t1 = u[j].y * scale_exp(rWi1 * cwi, f1 < cfm ? kExpOne : 0);
+        double r0 = rnd_int(t0), r1 = rnd_int(t1);
+        rd.words(t0, r0, t1, r1);
         if (j == j_sub) {
-          if (w_sub) r1 -= sub;
-          else r0 -= sub;
+          r0 -= two0;
+          r1 -= two1;
         }
-        const bool big0 = e0 < bb, big1 = e1 < bb;
-        const double P0 = big0 ? p2hi : p2lo, I0 = big0 ? ip2hi : ip2lo;
-        const double P1 = big1 ? p2hi : p2lo, I1 = big1 ? ip2hi : ip2lo;
-        const double h0 = rnd_int(r0 * I0), l0 = fma(-h0, P0, r0);
-        const double h1 = rnd_int(r1 * I1), l1 = fma(-h1, P1, r1);
-        const double tt1 = l1 + h0;
-        const double k1c = rnd_int(tt1 * I1);
-        const double d1p = fma(-k1c, P1, tt1);
-        const double co = h1 + k1c;
-        rw[m1] = make_double2(fma(d1p, 0x1p24, l0), co);
+        double pk, co;
+        carry_split(r0, r1, P0, I0, P1, I1, pk, co);
+        rw[m1] = make_double2(pk, co);
         if (row == RPC - 1) next_cin[wrap ? (m1 + 1 == W ? 0 : m1 + 1) : m1] = co;
       }
       // the carries of this CTA's rows are in place (the next row reads them
@@ -338,32 +329,26 @@ __global__ void __launch_bounds__(ClusterCfg<PR, TWR, PT, TC, C, RPC>::T, 1)
     if (wide) {
       // the first row waits for the previous CTA's carries (the only
       // dependence between CTAs inside the wide pass)
-      if (row == 0 && !mbar_wait(&s_cbar, it & 1u)) atomicOr(&s_fault, 1u);
+      if (row == 0 && !mbar_wait(&s_cbar, it & 1u)) atomicOr(&wa.st->fault, 1u);
       const bool last_it = report && it + 1 == iters;
       double2 x[EPR];
 #pragma unroll
       for (int j = 0; j < EPR; ++j) {
         const int m1 = t + j * TWR;
         const double c_in = row > 0 ? rows[(row - 1) * RS + m1].y : cin[m1];
-        const int cfm = cf[m1];
+        const uint32_t cfm = cf[m1];
         const double cw = cwt[m1].x;
-        int e0 = rE0 + cfm;
-        const bool f0 = e0 >= n, f1 = rE1 + cfm >= n;
-        if (f0) e0 -= n;
-        const bool big0 = e0 < bb;
-        const double P0 = big0 ? p2hi : p2lo, I0 = big0 ? ip2hi : ip2lo;
-        const double pk = rw[m1].x;
-        const double d1p = rnd_int(pk * 0x1p-24), l0 = fma(-d1p, 0x1p24, pk);
-        const double tt0 = l0 + c_in;
-        const double k0 = rnd_int(tt0 * I0);
-        const double d0 = fma(-k0, P0, tt0);
-        const double d1 = d1p + k0;
+        const uint32_t f0 = rF0 + cfm, f1 = rF1 + cfm;
+        double P0, I0, d0, d1;
+        ws.at(f0, P0, I0);
+        carry_join(rw[m1].x, c_in, P0, I0, d0, d1);
         if (last_it) {
           const uint32_t j0 = 2u * ((uint32_t)m1 * (uint32_t)H + (uint32_t)m2);
           wa.xint[j0] = (int32_t)d0;
           wa.xint[j0 + 1] = (int32_t)d1;
         }
-        x[j] = make_double2(d0 * (rW0 * cw * (f0 ? 0.5 : 1.0)), d1 * (rW1 * cw * (f1 ? 0.5 : 1.0)));
+        x[j] = make_double2(d0 * scale_exp(rW0 * cw, f0 < cfm ? -kExpOne : 0),
+                           d1 * scale_exp(rW1 * cw, f1 < cfm ? -kExpOne : 0));
       }
       // forward row transform: the first stage takes x[j] from registers
       // (its barrier orders the carry reads above before the row is
@@ -383,18 +368,5 @@ __global__ void __launch_bounds__(ClusterCfg<PR, TWR, PT, TC, C, RPC>::T, 1)
     ta.A[(size_t)cluster_col_k1<CF>(rank, lc) * H + m] = cols[lc * CS + pad(m)];
   }
   if (rank == 0 && tid == 0) ta.st->offset = off;
-  if (tid < TW) {
-    float em = (float)emax;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) em = fmaxf(em, __shfl_xor_sync(0xffffffffu, em, o));
-    if ((tid & 31) == 0) s_err[tid >> 5] = em;
-  }
-  if (out_of_range) atomicOr(&s_fault, 2u);
-  __syncthreads();
-  if (tid == 0 && rank < CF::ROWCTAS) {
-    float m = 0.f;
-    for (int i = 0; i < TW / 32; ++i) m = fmaxf(m, s_err[i]);
-    atomicMax(&wa.st->err_bits, __float_as_uint(m));
-    if (s_fault) atomicOr(&wa.st->fault, s_fault);
-  }
+  if (wide) rd.publish(wa.st, seen);
 }

@@ -634,13 +634,168 @@ __global__ void __launch_bounds__(2 * PP * TC, min_blocks(2 * PP * TC)) tall_any
 template <class P, int G>
 __host__ __device__ constexpr int wide_threads() { return G * (P::L / 16); }
 
-// Nearest integer of x for |x| < 2^51 (ties to even) by adding and removing
-// 1.5*2^52: two FP64 adds instead of a rounding instruction.  The _rn
-// intrinsics are never contracted or reassociated.  The carry splits below
-// apply it to values below 2^37 in magnitude.
-__device__ __forceinline__ double rnd_int(double x) {
-  return __dsub_rn(__dadd_rn(x, 6755399441055744.0), 6755399441055744.0);
+// Nearest integer of x * c for a power of two c, |x * c| < 2^51 (ties to
+// even), by adding and removing 1.5*2^52: the scaling is exact, so the fused
+// multiply-add rounds once, to the integer.  The _rn intrinsics are never
+// contracted or reassociated.
+constexpr double kRound = 6755399441055744.0;
+__device__ __forceinline__ double rnd_scaled(double x, double c) { return __dsub_rn(__fma_rn(x, c, kRound), kRound); }
+__device__ __forceinline__ double rnd_int(double x) { return __dsub_rn(__dadd_rn(x, kRound), kRound); }
+
+// x * 2^k through the exponent field (x normal, no over- or underflow).
+__device__ __forceinline__ double scale_exp(double x, int k20) {
+  return __hiloint2double(__double2hiint(x) + k20, __double2loint(x));
 }
+constexpr int kExpOne = 1 << 20;  // one step of the exponent field in the high word
+
+// The carry phases are latency bound in short passes (at 128K two warps per
+// SM spent 3.8 K of a row pass's 12.3 K cycles on phase 1): what counts is
+// their number of instructions.  Fractions that wrap by themselves, sizes and
+// wraps through the exponent field, integer maxima for the readings and
+// divisions by reciprocal took the pass from 4250 to 3850 instructions per
+// warp at 3200K, and 128K from 11.4 to 10.7 us per iteration, 512K from 15.3
+// to 14.7.
+//
+// Word sizes and weights.  The exponent e of a word's weight 2^(e/n) is kept
+// as the 32-bit fraction e/n + 1/(2n) of a turn: differences wrap by
+// themselves, and as n <= 2^25 the integers e lie 128 or more units apart, so
+// the rounding of the tables (one unit) never reaches a comparison, which all
+// fall half a step away from an integer.
+struct WordSize {
+  uint32_t lim;  // b/n: a word has qn + 1 bits where its fraction is below
+  int phi, ihi;  // high words of 2^qn and 2^-qn (the low words are zero)
+  __device__ __forceinline__ WordSize(uint32_t limit, int qn)
+      : lim(limit), phi((1023 + qn) << 20), ihi((1023 - qn) << 20) {}
+  __device__ __forceinline__ void at(uint32_t f, double &P, double &I) const {
+    const int k = f < lim ? kExpOne : 0;
+    P = __hiloint2double(phi + k, 0);
+    I = __hiloint2double(ihi - k, 0);
+  }
+};
+__device__ __forceinline__ uint32_t turn_fraction(int e, double turn) { return (uint32_t)fma((double)e, turn, 0.5 * turn); }
+
+// The readings of a thread's words: the largest |t - rint(t)| in units of
+// 2^-32 (an FP64 sum puts it into the low word, one integer maximum of three
+// takes it from there) and the largest magnitudes of t by its high word
+// (positive ones as signed, negative ones as unsigned integers).  At 2^51 and
+// above (or NaN) a double has no fraction bits left for the roundoff reading,
+// and the exact carry split no longer holds.
+struct Readings {
+  uint32_t err = 0, neg = 0;
+  int32_t pos = 0;
+  __device__ __forceinline__ void words(double t0, double r0, double t1, double r1) {
+    err = __vimax3_u32(err, (uint32_t)__double2loint(__dadd_rn(fabs(t0 - r0), 0x1p20)),
+                       (uint32_t)__double2loint(__dadd_rn(fabs(t1 - r1), 0x1p20)));
+    pos = __vimax3_s32(pos, __double2hiint(t0), __double2hiint(t1));
+    neg = __vimax3_u32(neg, (uint32_t)__double2hiint(t0), (uint32_t)__double2hiint(t1));
+  }
+  // Called by whole warps.  The device's maximum is touched only by a warp
+  // whose reading exceeds `seen`, its value read earlier in this pass (it
+  // only grows between the host's resets).
+  __device__ __forceinline__ void publish(DevState *st, uint32_t seen) {
+    const uint32_t e = __reduce_max_sync(0xffffffffu, err);
+    const bool out = pos >= 0x43200000 || neg >= 0xC3200000u;
+    const bool any = __any_sync(0xffffffffu, out);
+    if ((threadIdx.x & 31) == 0) {
+      const uint32_t bits = __float_as_uint((float)e * 0x1p-32f);
+      if (bits > seen) atomicMax(&st->err_bits, bits);
+      if (any) atomicOr(&st->fault, 2u);
+    }
+  }
+};
+
+// Phase 1 of the carry of an element with rounded words r0, r1: balanced
+// splits r = h*2^bits + l; word 1 takes high_0 and is balanced again.  The
+// outgoing carry h1 + (carry of that balance) depends on this element's own
+// words only.  pk packs l0 + d1p*2^24 (|l0|, |d1p| <= 2^(bits-1) < 2^23: exact
+// and separable).
+__device__ __forceinline__ void carry_split(double r0, double r1, double P0, double I0, double P1, double I1,
+                                            double &pk, double &co) {
+  const double h0 = rnd_scaled(r0, I0), l0 = fma(-h0, P0, r0);
+  const double h1 = rnd_scaled(r1, I1), l1 = fma(-h1, P1, r1);
+  const double tt1 = l1 + h0;
+  const double k1 = rnd_scaled(tt1, I1);
+  const double d1p = fma(-k1, P1, tt1);
+  co = h1 + k1;
+  pk = fma(d1p, 0x1p24, l0);
+}
+// Phase 2: the digits from the packed pair and the incoming carry.
+__device__ __forceinline__ void carry_join(double pk, double cin, double P0, double I0, double &d0, double &d1) {
+  const double d1p = rnd_scaled(pk, 0x1p-24), l0 = fma(-d1p, 0x1p24, pk);
+  const double tt0 = l0 + cin;
+  const double k0 = rnd_scaled(tt0, I0);
+  d0 = fma(-k0, P0, tt0);
+  d1 = d1p + k0;
+}
+
+// Carries between CTAs.  A published carry is a finite integer below 2^53, so
+// its slot in global memory says by itself whether it has come: empty slots
+// hold a value no carry has (kNoCarry, every byte 0x7F), and whoever takes a
+// carry empties the slot for the next iteration.  An eight-byte access is
+// single, so there is no flag, and no fence that would hold the publishing
+// warp until its stores are visible.  Per iteration, against flags released
+// and acquired per warp: 128K 10.7 -> 10.0 us, 512K 14.7 -> 13.5, 18432K
+// 385 -> 366, 3200K 62.2 -> 61.6.
+constexpr int kNoCarryByte = 0x7F, kNoCarryHi = 0x7F7F7F7F;
+__device__ __forceinline__ void put_carry(double *slot, double c) {
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(slot), "d"(c) : "memory");
+}
+__device__ __forceinline__ double peek_carry(const double *slot) {
+  double c;
+  asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(c) : "l"(slot) : "memory");
+  return c;
+}
+constexpr long long kWaitCycles = 2000000000;  // about a second
+// Takes R carries, slots at(r); the wait is bounded: on expiry it sets the
+// timeout fault bit and goes on.
+template <int R, class AT>
+__device__ __forceinline__ void take_carries(double *c, AT at, DevState *st) {
+  long long t0 = 0;
+  for (int k = 0;; ++k) {
+    bool missing = false;
+#pragma unroll
+    for (int r = 0; r < R; ++r) c[r] = peek_carry(at(r));
+#pragma unroll
+    for (int r = 0; r < R; ++r) missing |= __double2hiint(c[r]) == kNoCarryHi;
+    if (!missing) break;
+    const long long now = clock64();
+    if (k == 0) t0 = now;
+    else if (now - t0 > kWaitCycles || ((k & 1023) == 0 && (*(volatile uint32_t *)&st->fault & 1u))) {
+      atomicOr(&st->fault, 1u);
+      break;
+    }
+  }
+  const double none = __hiloint2double(kNoCarryHi, kNoCarryHi);
+#pragma unroll
+  for (int r = 0; r < R; ++r) put_carry(at(r), none);
+}
+
+// floor(x / d) for x < 2^58 and d < 2^31: an FP64 estimate (off by at most
+// one, its relative error is a few 2^-53 and the quotient is below 2^31),
+// then one exact correction step in integers.
+__device__ __forceinline__ uint32_t udiv_est(unsigned long long x, uint32_t d, double inv_d) {
+  unsigned long long e = (unsigned long long)((double)x * inv_d);
+  if (e * d > x) --e;
+  else if ((e + 1) * d <= x) ++e;
+  return (uint32_t)e;
+}
+
+// The -2 (bit (offset+1) mod q, CUDALucas.cu:1882-1886) hits one word: the
+// element (m1, m2) that holds it, and what its two words lose.
+struct MinusTwo {
+  uint32_t m1, m2;
+  double s0, s1;
+  __device__ __forceinline__ MinusTwo(uint32_t offset, const WideArgs &a) {
+    const uint32_t pos = offset + 1 == a.q ? 0u : offset + 1;
+    const uint32_t dw = udiv_est((unsigned long long)pos * a.n, a.q, a.inv_q);
+    const uint32_t sdw = udiv_est((unsigned long long)dw * a.q + a.n - 1, a.n, a.inv_n);
+    m1 = udiv_est(dw >> 1, (uint32_t)a.H, a.inv_H);
+    m2 = (dw >> 1) - m1 * (uint32_t)a.H;
+    const double sub = __hiloint2double((1023 + (int)(pos - sdw)) << 20, 0);
+    s0 = dw & 1 ? 0.0 : sub;
+    s1 = dw & 1 ? sub : 0.0;
+  }
+};
 
 // Wide pass for rows of length W = P::L; G rows per CTA.
 // The carry arithmetic runs in FP64 on integer-valued doubles (all values
@@ -656,10 +811,7 @@ __device__ __forceinline__ void wide_body(const WideArgs &a, int blk, S sync = S
   constexpr int RS = row_slots<W, G>();
   double2 *stw = sm + G * RS;
   __shared__ int s_g;
-  __shared__ float s_err[32];
-  __shared__ uint32_t s_fault;
   if (threadIdx.x == 0) {
-    s_fault = 0;
     s_g = MODE == WIDE_INIT ? (BATCH ? blk : (int)blockIdx.x)
                             : (int)(atomicAdd(&a.st->ticket, 1ull) % (unsigned long long)a.ngroups);
   }
@@ -676,33 +828,33 @@ __device__ __forceinline__ void wide_body(const WideArgs &a, int blk, S sync = S
   constexpr bool kDirect = G > 1;
   const int row = threadIdx.x % G, t = threadIdx.x / G;
   const int m2 = m2b + row;
-  const int n = (int)a.n, bb = (int)a.b, qn = (int)a.qn;
+  const int n = (int)a.n;
   // Word s (0, 1) of element (m1 = t + r*TR, m2) has weight exponent
-  // e = (E_s - colD[r]) mod n with the per-thread E_s = rowE + colF[t] mod n,
-  // so its weight is Wt_s * colS[r] (or * colS2[r] when E_s < colD[r]).
+  // e = (E_s - D_r) mod n with the per-thread E_s = rowE + colF[t] mod n, so
+  // its weight is W_s * colS[r], doubled when E_s < D_r.
   int E0 = __ldg(&a.rowE[2 * m2]) + __ldg(&a.colF[t]);
   int E1 = __ldg(&a.rowE[2 * m2 + 1]) + __ldg(&a.colF[t]);
+  const bool w0 = E0 >= n, w1 = E1 >= n;
+  if (w0) E0 -= n;
+  if (w1) E1 -= n;
   const double cwt = __ldg(&a.colW[t]);
-  const double W0 = __ldg(&a.rowW[2 * m2]) * cwt * (E0 >= n ? 0.5 : 1.0);
-  const double W1 = __ldg(&a.rowW[2 * m2 + 1]) * cwt * (E1 >= n ? 0.5 : 1.0);
-  if (E0 >= n) E0 -= n;
-  if (E1 >= n) E1 -= n;
-  const double p2lo = (double)(1 << qn), p2hi = 2.0 * p2lo;
-  const double ip2lo = 1.0 / p2lo, ip2hi = 0.5 * ip2lo;
-  double2 x[16];
-  double emax = 0.0;
-  bool out_of_range = false;
+  const double W0 = __ldg(&a.rowW[2 * m2]) * cwt * (w0 ? 0.5 : 1.0);
+  const double W1 = __ldg(&a.rowW[2 * m2 + 1]) * cwt * (w1 ? 0.5 : 1.0);
   double Wi0 = 0.0, Wi1 = 0.0;
   if (MODE != WIDE_INIT) {
     const double cwit = __ldg(&a.colWi[t]);
-    Wi0 = __ldg(&a.rowWi[2 * m2]) * cwit * (__ldg(&a.rowE[2 * m2]) + __ldg(&a.colF[t]) >= n ? 2.0 : 1.0);
-    Wi1 = __ldg(&a.rowWi[2 * m2 + 1]) * cwit * (__ldg(&a.rowE[2 * m2 + 1]) + __ldg(&a.colF[t]) >= n ? 2.0 : 1.0);
+    Wi0 = __ldg(&a.rowWi[2 * m2]) * cwit * (w0 ? 2.0 : 1.0);
+    Wi1 = __ldg(&a.rowWi[2 * m2 + 1]) * cwit * (w1 ? 2.0 : 1.0);
   }
+  const uint32_t F0 = turn_fraction(E0, a.turn), F1 = turn_fraction(E1, a.turn);
+  const WordSize ws(a.lim, (int)a.qn);
+  double2 x[16];
   // everything above reads constant tables only; the state array, the
   // digits and the device state are read after the previous pass completed
   griddep_wait();
   griddep_release();
   if (MODE != WIDE_INIT) {
+    const uint32_t off = __ldcg(&a.st->offset), seen = __ldcg(&a.st->err_bits);
     if constexpr (kDirect) {
       // the inverse transform's first stage (radix 16, no twiddle) works on
       // elements t + r*TR of the row: straight from global memory
@@ -721,19 +873,9 @@ __device__ __forceinline__ void wide_body(const WideArgs &a, int blk, S sync = S
 #pragma unroll
       for (int r = 0; r < 16; ++r) prefetch_l2(nxt + (size_t)(t + r * TR) * H);
     }
-    // the -2 (bit (offset+1) mod q, CUDALucas.cu:1882-1886) hits at most one
-    // word; locate it once: element register r_sub, word w_sub
-    const uint32_t off = a.st->offset;
-    const uint32_t pos = (off + 1) % a.q;
-    const uint32_t dw = (uint32_t)(((unsigned long long)pos * a.n) / a.q);
-    const uint32_t sdw = (uint32_t)(((unsigned long long)dw * a.q + a.n - 1) / a.n);
-    const double sub = (double)(1u << (pos - sdw));
-    int r_sub = -1;
-    {
-      const uint32_t me = dw >> 1, mm1 = me / (uint32_t)H, mm2 = me - mm1 * (uint32_t)H;
-      if ((int)mm2 == m2 && (int)(mm1 % TR) == t) r_sub = (int)(mm1 / TR);
-    }
-    const bool w_sub = dw & 1;
+    // element register of this thread that the -2 hits, if any
+    const MinusTwo two(off, a);
+    const int r_sub = (int)two.m2 == m2 && (int)(two.m1 % TR) == t ? (int)(two.m1 / TR) : -1;
     cp_async_wait_all();
     sync();
     if constexpr (kDirect) inv_stages<P, RS, 1, P::N - 1, 16, TR>(sm, stw, row, t, sync);
@@ -742,97 +884,62 @@ __device__ __forceinline__ void wide_body(const WideArgs &a, int blk, S sync = S
     last_stage_to_regs<W, RS, TR>(sm, stw + tw_offset<P, P::N - 1>(), u, row, t);
     sync();  // shared memory is reused for the carry hand-off below
 
-    // Carry in FP64 only (no integer conversions).  Phase 1 leaves, in the
-    // shared-memory slot of element (row, m1), the packed pair
-    // l0 + d1p*2^24 (|l0|, |d1p| <= 2^(bits-1) < 2^23, so the pair is exact
-    // and separable) and the element's outgoing carry.
+    // Phase 1 of the carry leaves, in the shared-memory slot of element
+    // (row, m1), the packed pair of carry_split and the outgoing carry.
     double2 *ks = sm + row * RS + t;  // ks[r*TR]: element m1 = t + r*TR
     double *gcd = reinterpret_cast<double *>(a.carry);
+    Readings rd;
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
-      const int m1 = t + r * TR;
-      const int D = a.colD[r];
-      const bool n0 = E0 < D, n1 = E1 < D;
-      const int e0 = E0 - D + (n0 ? n : 0), e1 = E1 - D + (n1 ? n : 0);
-      const double t0 = u[r].x * (Wi0 * (n0 ? a.colSi2[r] : a.colSi[r]));
-      const double t1 = u[r].y * (Wi1 * (n1 ? a.colSi2[r] : a.colSi[r]));
-      double r0 = rint(t0), r1 = rint(t1);
-      emax = fmax(emax, fmax(fabs(t0 - r0), fabs(t1 - r1)));
-      // at 2^51 and above (or NaN) a double has no fraction bits left for the
-      // roundoff reading, and the exact carry split below no longer holds
-      if (!(fabs(t0) < 0x1p51 && fabs(t1) < 0x1p51)) out_of_range = true;
+      const uint32_t D = a.colD[r];
+      double P0, I0, P1, I1;
+      ws.at(F0 - D, P0, I0);
+      ws.at(F1 - D, P1, I1);
+      const double t0 = u[r].x * scale_exp(Wi0 * a.colSi[r], F0 < D ? -kExpOne : 0);
+      const double t1 = u[r].y * scale_exp(Wi1 * a.colSi[r], F1 < D ? -kExpOne : 0);
+      double r0 = rnd_int(t0), r1 = rnd_int(t1);
+      rd.words(t0, r0, t1, r1);
       if (r == r_sub) {
-        if (w_sub) r1 -= sub;
-        else r0 -= sub;
+        r0 -= two.s0;
+        r1 -= two.s1;
       }
-      const bool big0 = e0 < bb, big1 = e1 < bb;
-      const double P0 = big0 ? p2hi : p2lo, I0 = big0 ? ip2hi : ip2lo;
-      const double P1 = big1 ? p2hi : p2lo, I1 = big1 ? ip2hi : ip2lo;
-      // balanced splits r = h*2^bits + l; word 1 takes high_0 and is
-      // balanced again; the outgoing carry high_1 + (carry of that balance)
-      // depends on this element's own words only
-      const double h0 = rnd_int(r0 * I0), l0 = fma(-h0, P0, r0);
-      const double h1 = rnd_int(r1 * I1), l1 = fma(-h1, P1, r1);
-      const double tt1 = l1 + h0;
-      const double k1c = rnd_int(tt1 * I1);
-      const double d1p = fma(-k1c, P1, tt1);
-      const double co = h1 + k1c;
-      ks[r * TR] = make_double2(fma(d1p, 0x1p24, l0), co);
-      if (row == G - 1) gcd[(size_t)g * W + m1] = co;
+      double pk, co;
+      carry_split(r0, r1, P0, I0, P1, I1, pk, co);
+      ks[r * TR] = make_double2(pk, co);
+      if (row == G - 1) put_carry(&gcd[(size_t)g * W + t + r * TR], co);
     }
-    // Hand-off warp by warp: warp w holds the same element columns m1 in
-    // every CTA, so it publishes its last row's carries with its own flag
-    // and waits only for the flag of warp w of the predecessor.  __syncwarp
-    // orders the lanes' stores and loads around lane 0's release store and
-    // acquire load.  (The wrap into CTA 0 shifts m1 by one across warps, so
-    // CTA 0 waits for all warps of the last CTA.)
+    rd.publish(a.st, seen);
+    // The G rows of an element column sit in adjacent lanes: rows above the
+    // first take the carries of the row before from its slots, the first row
+    // those that the CTA before has put into global memory (into CTA 0 shifted
+    // by one element).
     const int pred = g == 0 ? a.ngroups - 1 : g - 1;
-    constexpr int NW = T / 32;
-    static_assert(T % 32 == 0 && NW <= kWarpFlags, "whole warps, one flag each");
-    const int warp = threadIdx.x >> 5;
+    static_assert(T % 32 == 0, "whole warps");
     __syncwarp();
-    if ((threadIdx.x & 31) == 0)
-      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&a.flags[g * kWarpFlags + warp]), "r"(1u) : "memory");
-    if (g != 0) {
-      if ((threadIdx.x & 31) == 0) {
-        uint32_t *f = &a.flags[pred * kWarpFlags + warp];
-        if (!wait_flag(f)) atomicOr(&s_fault, 1u);
-        *f = 0;
-      }
-      __syncwarp();
+    double cin[16];
+    if (row > 0) {
+#pragma unroll
+      for (int r = 0; r < 16; ++r) cin[r] = sm[(row - 1) * RS + t + r * TR].y;
     } else {
-      sync();
-      if (threadIdx.x == 0) {
-        for (int w = 0; w < NW; ++w) {
-          uint32_t *f = &a.flags[pred * kWarpFlags + w];
-          if (!wait_flag(f)) s_fault |= 1u;
-          *f = 0;
-        }
-      }
-      sync();
+      double *in = gcd + (size_t)pred * W;
+      take_carries<16>(cin, [&](int r) {
+        const int m1 = t + r * TR;
+        return in + (g == 0 ? (m1 == 0 ? W - 1 : m1 - 1) : m1);
+      }, a.st);
     }
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
-      const int m1 = t + r * TR;
-      const double cin = row > 0 ? sm[(row - 1) * RS + m1].y
-                                 : __ldcg(&gcd[(size_t)pred * W + (g == 0 ? (m1 == 0 ? W - 1 : m1 - 1) : m1)]);
-      const int D = a.colD[r];
-      const bool n0 = E0 < D, n1 = E1 < D;
-      const int e0 = E0 - D + (n0 ? n : 0);
-      const bool big0 = e0 < bb;
-      const double P0 = big0 ? p2hi : p2lo, I0 = big0 ? ip2hi : ip2lo;
-      const double pk = ks[r * TR].x;
-      const double d1p = rnd_int(pk * 0x1p-24), l0 = fma(-d1p, 0x1p24, pk);
-      const double tt0 = l0 + cin;
-      const double k0 = rnd_int(tt0 * I0);
-      const double d0 = fma(-k0, P0, tt0);
-      const double d1 = d1p + k0;
+      const uint32_t D = a.colD[r];
+      double P0, I0, d0, d1;
+      ws.at(F0 - D, P0, I0);
+      carry_join(ks[r * TR].x, cin[r], P0, I0, d0, d1);
       if (MODE == WIDE_REPORT) {
-        const uint32_t j0 = 2u * ((uint32_t)m1 * (uint32_t)H + (uint32_t)m2);
+        const uint32_t j0 = 2u * ((uint32_t)(t + r * TR) * (uint32_t)H + (uint32_t)m2);
         a.xint[j0] = (int32_t)d0;
         a.xint[j0 + 1] = (int32_t)d1;
       }
-      x[r] = make_double2(d0 * (W0 * (n0 ? a.colS2[r] : a.colS[r])), d1 * (W1 * (n1 ? a.colS2[r] : a.colS[r])));
+      x[r] = make_double2(d0 * scale_exp(W0 * a.colS[r], F0 < D ? kExpOne : 0),
+                          d1 * scale_exp(W1 * a.colS[r], F1 < D ? kExpOne : 0));
     }
     sync();  // carry reads done before the data region is rewritten
   } else {
@@ -840,12 +947,10 @@ __device__ __forceinline__ void wide_body(const WideArgs &a, int blk, S sync = S
     sync();
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
-      const int m1 = t + r * TR;
-      const int D = a.colD[r];
-      const bool n0 = E0 < D, n1 = E1 < D;
-      const uint32_t j0 = 2u * ((uint32_t)m1 * (uint32_t)H + (uint32_t)m2);
-      x[r] = make_double2((double)a.xint[j0] * (W0 * (n0 ? a.colS2[r] : a.colS[r])),
-                          (double)a.xint[j0 + 1] * (W1 * (n1 ? a.colS2[r] : a.colS[r])));
+      const uint32_t D = a.colD[r];
+      const uint32_t j0 = 2u * ((uint32_t)(t + r * TR) * (uint32_t)H + (uint32_t)m2);
+      x[r] = make_double2((double)a.xint[j0] * scale_exp(W0 * a.colS[r], F0 < D ? kExpOne : 0),
+                          (double)a.xint[j0 + 1] * scale_exp(W1 * a.colS[r], F1 < D ? kExpOne : 0));
     }
   }
   first_stage_from_regs<W, RS, TR>(sm, x, row, t);
@@ -861,20 +966,6 @@ __device__ __forceinline__ void wide_body(const WideArgs &a, int blk, S sync = S
   } else {
     fwd_stages<P, RS, 1, P::N, 16, TR>(sm, stw, row, t, sync);
     for (int k1 = threadIdx.x; k1 < W; k1 += T) a.A[(size_t)k1 * H + m2b] = sm[pad(k1)];
-  }
-  if (MODE != WIDE_INIT) {
-    float em = (float)emax;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) em = fmaxf(em, __shfl_xor_sync(0xffffffffu, em, o));
-    if ((threadIdx.x & 31) == 0) s_err[threadIdx.x >> 5] = em;
-    if (out_of_range) atomicOr(&s_fault, 2u);
-    sync();
-    if (threadIdx.x == 0) {
-      float m = 0.f;
-      for (int i = 0; i < (T + 31) / 32; ++i) m = fmaxf(m, s_err[i]);
-      atomicMax(&a.st->err_bits, __float_as_uint(m));
-      if (s_fault) atomicOr(&a.st->fault, s_fault);
-    }
   }
 }
 
@@ -903,10 +994,7 @@ __device__ __forceinline__ void wide_any_body(const WideArgs &a, int blk, S sync
   constexpr int RS = row_slots<W, G>();
   double2 *stw = sm + G * RS;
   __shared__ int s_g;
-  __shared__ float s_err[32];
-  __shared__ uint32_t s_fault;
   if (threadIdx.x == 0) {
-    s_fault = 0;
     s_g = MODE == WIDE_INIT ? (BATCH ? blk : (int)blockIdx.x)
                             : (int)(atomicAdd(&a.st->ticket, 1ull) % (unsigned long long)a.ngroups);
   }
@@ -917,46 +1005,36 @@ __device__ __forceinline__ void wide_any_body(const WideArgs &a, int blk, S sync
   const int m2b = g * G;
   const int row = threadIdx.x % G, t = threadIdx.x / G;
   const int m2 = m2b + row;
-  const int n = (int)a.n, bb = (int)a.b, qn = (int)a.qn;
+  const int n = (int)a.n;
   int E0 = __ldg(&a.rowE[2 * m2]) + __ldg(&a.colF[t]);
   int E1 = __ldg(&a.rowE[2 * m2 + 1]) + __ldg(&a.colF[t]);
+  const bool w0 = E0 >= n, w1 = E1 >= n;
+  if (w0) E0 -= n;
+  if (w1) E1 -= n;
   const double cwt = __ldg(&a.colW[t]);
-  const double W0 = __ldg(&a.rowW[2 * m2]) * cwt * (E0 >= n ? 0.5 : 1.0);
-  const double W1 = __ldg(&a.rowW[2 * m2 + 1]) * cwt * (E1 >= n ? 0.5 : 1.0);
+  const double W0 = __ldg(&a.rowW[2 * m2]) * cwt * (w0 ? 0.5 : 1.0);
+  const double W1 = __ldg(&a.rowW[2 * m2 + 1]) * cwt * (w1 ? 0.5 : 1.0);
   double Wi0 = 0.0, Wi1 = 0.0;
   if (MODE != WIDE_INIT) {
     const double cwit = __ldg(&a.colWi[t]);
-    Wi0 = __ldg(&a.rowWi[2 * m2]) * cwit * (E0 >= n ? 2.0 : 1.0);
-    Wi1 = __ldg(&a.rowWi[2 * m2 + 1]) * cwit * (E1 >= n ? 2.0 : 1.0);
+    Wi0 = __ldg(&a.rowWi[2 * m2]) * cwit * (w0 ? 2.0 : 1.0);
+    Wi1 = __ldg(&a.rowWi[2 * m2 + 1]) * cwit * (w1 ? 2.0 : 1.0);
   }
-  if (E0 >= n) E0 -= n;
-  if (E1 >= n) E1 -= n;
-  const double p2lo = (double)(1 << qn), p2hi = 2.0 * p2lo;
-  const double ip2lo = 1.0 / p2lo, ip2hi = 0.5 * ip2lo;
+  const uint32_t F0 = turn_fraction(E0, a.turn), F1 = turn_fraction(E1, a.turn);
+  const WordSize ws(a.lim, (int)a.qn);
   double2 *rw = sm + row * RS;
   auto ld = [&](int e, int, int) { return rw[pad(e)]; };
   auto st = [&](int e, int, int, double2 v) { rw[pad(e)] = v; };
   double2 x[R];
-  double emax = 0.0;
-  bool out_of_range = false;
   // everything above reads constant tables only; the state array, the
   // digits and the device state are read after the previous pass completed
   griddep_wait();
   griddep_release();
   if (MODE != WIDE_INIT) {
-    // the -2 (bit (offset+1) mod q, CUDALucas.cu:1882-1886) hits at most one
-    // word; locate it once: element register r_sub, word w_sub
-    const uint32_t off = a.st->offset;
-    const uint32_t pos = (off + 1) % a.q;
-    const uint32_t dw = (uint32_t)(((unsigned long long)pos * a.n) / a.q);
-    const uint32_t sdw = (uint32_t)(((unsigned long long)dw * a.q + a.n - 1) / a.n);
-    const double sub = (double)(1u << (pos - sdw));
-    int r_sub = -1;
-    {
-      const uint32_t me = dw >> 1, mm1 = me / (uint32_t)H, mm2 = me - mm1 * (uint32_t)H;
-      if ((int)mm2 == m2 && (int)(mm1 % TR) == t) r_sub = (int)(mm1 / TR);
-    }
-    const bool w_sub = dw & 1;
+    const uint32_t off = __ldcg(&a.st->offset), seen = __ldcg(&a.st->err_bits);
+    // element register of this thread that the -2 hits, if any
+    const MinusTwo two(off, a);
+    const int r_sub = (int)two.m2 == m2 && (int)(two.m1 % TR) == t ? (int)(two.m1 / TR) : -1;
     // inverse row transform: the first stage straight from global memory,
     // the last into registers (elements t + r*TR)
     const double2 *src = a.A + m2;
@@ -967,92 +1045,67 @@ __device__ __forceinline__ void wide_any_body(const WideArgs &a, int blk, S sync
     fall_stages<P, 0, 1, TR, -1, false, false>(stw, t, sync, ld_first, st_reg, ld, st);
     double2 *ks = rw + t;  // ks[r*TR]: element m1 = t + r*TR
     double *gcd = reinterpret_cast<double *>(a.carry);
+    Readings rd;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int m1 = t + r * TR;
-      const int D = a.colD[r];
-      const bool n0 = E0 < D, n1 = E1 < D;
-      const int e0 = E0 - D + (n0 ? n : 0), e1 = E1 - D + (n1 ? n : 0);
-      const double t0 = u[r].x * (Wi0 * (n0 ? a.colSi2[r] : a.colSi[r]));
-      const double t1 = u[r].y * (Wi1 * (n1 ? a.colSi2[r] : a.colSi[r]));
-      double r0 = rint(t0), r1 = rint(t1);
-      emax = fmax(emax, fmax(fabs(t0 - r0), fabs(t1 - r1)));
-      if (!(fabs(t0) < 0x1p51 && fabs(t1) < 0x1p51)) out_of_range = true;
+      const uint32_t D = a.colD[r];
+      double P0, I0, P1, I1;
+      ws.at(F0 - D, P0, I0);
+      ws.at(F1 - D, P1, I1);
+      const double t0 = u[r].x * scale_exp(Wi0 * a.colSi[r], F0 < D ? -kExpOne : 0);
+      const double t1 = u[r].y * scale_exp(Wi1 * a.colSi[r], F1 < D ? -kExpOne : 0);
+      double r0 = rnd_int(t0), r1 = rnd_int(t1);
+      rd.words(t0, r0, t1, r1);
       if (r == r_sub) {
-        if (w_sub) r1 -= sub;
-        else r0 -= sub;
+        r0 -= two.s0;
+        r1 -= two.s1;
       }
-      const bool big0 = e0 < bb, big1 = e1 < bb;
-      const double P0 = big0 ? p2hi : p2lo, I0 = big0 ? ip2hi : ip2lo;
-      const double P1 = big1 ? p2hi : p2lo, I1 = big1 ? ip2hi : ip2lo;
-      const double h0 = rnd_int(r0 * I0), l0 = fma(-h0, P0, r0);
-      const double h1 = rnd_int(r1 * I1), l1 = fma(-h1, P1, r1);
-      const double tt1 = l1 + h0;
-      const double k1c = rnd_int(tt1 * I1);
-      const double d1p = fma(-k1c, P1, tt1);
-      const double co = h1 + k1c;
-      ks[r * TR] = make_double2(fma(d1p, 0x1p24, l0), co);
-      if (row == G - 1) gcd[(size_t)g * W + m1] = co;
+      double pk, co;
+      carry_split(r0, r1, P0, I0, P1, I1, pk, co);
+      ks[r * TR] = make_double2(pk, co);
+      if (row == G - 1) put_carry(&gcd[(size_t)g * W + t + r * TR], co);
     }
-    // hand-off warp by warp, as in wide_body
+    rd.publish(a.st, seen);
+    // The G rows of an element column sit in adjacent lanes: rows above the
+    // first take the carries of the row before from its slots, the first row
+    // those that the CTA before has put into global memory (into CTA 0 shifted
+    // by one element).
     const int pred = g == 0 ? a.ngroups - 1 : g - 1;
-    constexpr int NW = T / 32;
-    static_assert(T % 32 == 0 && NW <= kWarpFlags, "whole warps, one flag each");
-    const int warp = threadIdx.x >> 5;
+    static_assert(T % 32 == 0, "whole warps");
     __syncwarp();
-    if ((threadIdx.x & 31) == 0)
-      asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&a.flags[g * kWarpFlags + warp]), "r"(1u) : "memory");
-    if (g != 0) {
-      if ((threadIdx.x & 31) == 0) {
-        uint32_t *f = &a.flags[pred * kWarpFlags + warp];
-        if (!wait_flag(f)) atomicOr(&s_fault, 1u);
-        *f = 0;
-      }
-      __syncwarp();
+    double cin[R];
+    if (row > 0) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) cin[r] = sm[(row - 1) * RS + t + r * TR].y;
     } else {
-      sync();
-      if (threadIdx.x == 0) {
-        for (int w = 0; w < NW; ++w) {
-          uint32_t *f = &a.flags[pred * kWarpFlags + w];
-          if (!wait_flag(f)) s_fault |= 1u;
-          *f = 0;
-        }
-      }
-      sync();
+      double *in = gcd + (size_t)pred * W;
+      take_carries<R>(cin, [&](int r) {
+        const int m1 = t + r * TR;
+        return in + (g == 0 ? (m1 == 0 ? W - 1 : m1 - 1) : m1);
+      }, a.st);
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int m1 = t + r * TR;
-      const double cin = row > 0 ? sm[(row - 1) * RS + m1].y
-                                 : __ldcg(&gcd[(size_t)pred * W + (g == 0 ? (m1 == 0 ? W - 1 : m1 - 1) : m1)]);
-      const int D = a.colD[r];
-      const bool n0 = E0 < D, n1 = E1 < D;
-      const int e0 = E0 - D + (n0 ? n : 0);
-      const bool big0 = e0 < bb;
-      const double P0 = big0 ? p2hi : p2lo, I0 = big0 ? ip2hi : ip2lo;
-      const double pk = ks[r * TR].x;
-      const double d1p = rnd_int(pk * 0x1p-24), l0 = fma(-d1p, 0x1p24, pk);
-      const double tt0 = l0 + cin;
-      const double k0 = rnd_int(tt0 * I0);
-      const double d0 = fma(-k0, P0, tt0);
-      const double d1 = d1p + k0;
+      const uint32_t D = a.colD[r];
+      double P0, I0, d0, d1;
+      ws.at(F0 - D, P0, I0);
+      carry_join(ks[r * TR].x, cin[r], P0, I0, d0, d1);
       if (MODE == WIDE_REPORT) {
-        const uint32_t j0 = 2u * ((uint32_t)m1 * (uint32_t)H + (uint32_t)m2);
+        const uint32_t j0 = 2u * ((uint32_t)(t + r * TR) * (uint32_t)H + (uint32_t)m2);
         a.xint[j0] = (int32_t)d0;
         a.xint[j0 + 1] = (int32_t)d1;
       }
-      x[r] = make_double2(d0 * (W0 * (n0 ? a.colS2[r] : a.colS[r])), d1 * (W1 * (n1 ? a.colS2[r] : a.colS[r])));
+      x[r] = make_double2(d0 * scale_exp(W0 * a.colS[r], F0 < D ? kExpOne : 0),
+                          d1 * scale_exp(W1 * a.colS[r], F1 < D ? kExpOne : 0));
     }
   } else {
     cp_async_wait_all();
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const int m1 = t + r * TR;
-      const int D = a.colD[r];
-      const bool n0 = E0 < D, n1 = E1 < D;
-      const uint32_t j0 = 2u * ((uint32_t)m1 * (uint32_t)H + (uint32_t)m2);
-      x[r] = make_double2((double)a.xint[j0] * (W0 * (n0 ? a.colS2[r] : a.colS[r])),
-                          (double)a.xint[j0 + 1] * (W1 * (n1 ? a.colS2[r] : a.colS[r])));
+      const uint32_t D = a.colD[r];
+      const uint32_t j0 = 2u * ((uint32_t)(t + r * TR) * (uint32_t)H + (uint32_t)m2);
+      x[r] = make_double2((double)a.xint[j0] * scale_exp(W0 * a.colS[r], F0 < D ? kExpOne : 0),
+                          (double)a.xint[j0 + 1] * scale_exp(W1 * a.colS[r], F1 < D ? kExpOne : 0));
     }
   }
   // forward row transform: the first stage from registers (its barrier
@@ -1062,20 +1115,6 @@ __device__ __forceinline__ void wide_any_body(const WideArgs &a, int blk, S sync
   auto ld_reg = [&](int, int, int r) { return x[r]; };
   auto st_last = [&](int e, int, int, double2 v) { dst[(size_t)e * H] = v; };
   fall_stages<P, 0, 1, TR, +1, true, false>(stw, t, sync, ld_reg, st_last, ld, st);
-  if (MODE != WIDE_INIT) {
-    float em = (float)emax;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) em = fmaxf(em, __shfl_xor_sync(0xffffffffu, em, o));
-    if ((threadIdx.x & 31) == 0) s_err[threadIdx.x >> 5] = em;
-    if (out_of_range) atomicOr(&s_fault, 2u);
-    sync();
-    if (threadIdx.x == 0) {
-      float m = 0.f;
-      for (int i = 0; i < (T + 31) / 32; ++i) m = fmaxf(m, s_err[i]);
-      atomicMax(&a.st->err_bits, __float_as_uint(m));
-      if (s_fault) atomicOr(&a.st->fault, s_fault);
-    }
-  }
 }
 
 template <class P, int G>
