@@ -423,11 +423,11 @@ struct StaticTall {
 // solo launches: members without one run on their own branch)
 #define LLB_TALL_ANY_SOLO(LIST, TC, PP)                                                                  \
   {LIST::L, tall_any<LIST, TC, PP>, nullptr, LLB_RAD(LIST), tw_size<LIST>(),                               \
-   tall_any_smem<LIST, PP>(), 2 * PP * TC, PP}
+   tall_any_smem<LIST, TC, PP>(), 2 * PP * TC, PP}
 // any radix list: TC threads per column, PP column pairs per CTA
 #define LLB_TALL_ANY(LIST, TC, PP)                                                                       \
   {LIST::L, tall_any<LIST, TC, PP>, tall_any_batch<LIST, TC, PP>, LLB_RAD(LIST), tw_size<LIST>(),          \
-   tall_any_smem<LIST, PP>(), 2 * PP * TC, PP}
+   tall_any_smem<LIST, TC, PP>(), 2 * PP * TC, PP}
 
 using L256 = RList<16, 16>;
 using L512 = RList<16, 2, 16>;
@@ -584,7 +584,7 @@ struct FusedKernel {
   {LW::L, LT::L, G, fused_iters<LW, G, FusedTall<LT, TC, PP>>, fused_threads<LW, G, FusedTall<LT, TC, PP>>(), \
    TC ? PP : 1,                                                                                              \
    std::max(G * row_slots<LW::L, G>() + tw_size<LW>(),                                                     \
-            TC ? tall_any_smem<LT, PP>() : padded(2 * LT::L) + tall_extra<LT>())}
+            TC ? tall_any_smem<LT, TC ? TC : 1, PP>() : padded(2 * LT::L) + tall_extra<LT>())}
 static const FusedKernel kFused[] = {
     LLB_FUSED(L256, 2, C24, 6, 8),
     LLB_FUSED(L256, 2, C28, 7, 16),

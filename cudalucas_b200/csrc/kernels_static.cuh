@@ -228,8 +228,10 @@ constexpr int tall_threads() { return 2 * (P::L / 16); }
 
 // Blocks per SM to ask of the register allocator: about 128 registers per
 // thread, which leaves room for two or more CTAs per SM.
+// (whole warps: a CTA of 20 threads holds the registers of 32).
 constexpr int min_blocks(int threads) {
-  return 65536 / (threads * 128) > 32 ? 32 : 65536 / (threads * 128) > 1 ? 65536 / (threads * 128) : 1;
+  const int b = 65536 / ((threads + 31) / 32 * 32 * 128);
+  return b > 1 ? b : 1;
 }
 
 // Shared memory of the tall pass beyond the two columns: stage twiddles,
@@ -276,7 +278,7 @@ __host__ __device__ constexpr bool tall_half_exchange() { return (P::L / 16) % 3
 
 template <class P>
 __host__ __device__ constexpr int tall_extra() {
-  return tw_size<P>() + 32 + 8 + (tall_half_exchange<P>() ? 16 + 4 * (P::L / 16) : 0);
+  return tw_size<P>() + 32 + 8 + (tall_half_exchange<P>() ? 16 + 4 * (P::L / 16) : 4 * (P::L / 16));
 }
 
 // Tall pass for columns of length H = P::L (radix list 16, M, 16 or 16, 16); two
@@ -305,6 +307,7 @@ __device__ __forceinline__ void tall_body(const TallArgs &a, int blk, S sync = S
   double2 *fr = pj + 8;              // w_H^(r*TR), half exchange
   double2 *sbase = fr + 16;          // per thread: w_N^(k1*t), half exchange
   double2 *spair = sbase + T;        // per thread: w_N^kA * w_H^tA, half exchange
+  double2 *sidx = pj + 8;            // per thread: w_H^i and w_N^kb * w_H^i, pairing by index
   const int c = blk;
   const int W = a.W;
   const bool special = (c == 0);
@@ -330,6 +333,12 @@ __device__ __forceinline__ void tall_body(const TallArgs &a, int blk, S sync = S
   if constexpr (kHalf) {
     sbase[threadIdx.x] = base;
     spair[threadIdx.x] = cmul(omegaN(a.thi, a.tlo, a.ts, a.tmask, kA), __ldg(&a.twH[col ? TR - 1 - t : t]));
+  } else {
+    // the table loads of the pairing come before the wait for the previous
+    // pass (128K: 1.9 K of the pass's 5.7 K cycles were the pairing)
+    const double2 wt = __ldg(&a.twH[threadIdx.x]);
+    sidx[threadIdx.x] = wt;
+    sidx[T + threadIdx.x] = cmul(omegaN(a.thi, a.tlo, a.ts, a.tmask, special ? W / 2 : kA), wt);
   }
   griddep_wait();
   griddep_release();
@@ -386,9 +395,15 @@ __device__ __forceinline__ void tall_body(const TallArgs &a, int blk, S sync = S
     for (int r = 0; r < 16; ++r) own[pad(t + r * TR)] = o[r];
     sync();
     // pairing by index: i = threadIdx.x + j*T, w_H^i = w_H^threadIdx.x * pj[j]
-    const double2 wt = __ldg(&a.twH[threadIdx.x]);
+    double2 wt, wb;
+    if constexpr (kHalf) {  // (pair 0 only)
+      wt = __ldg(&a.twH[threadIdx.x]);
+      wb = cmul(omegaN(a.thi, a.tlo, a.ts, a.tmask, W / 2), wt);
+    } else {
+      wt = sidx[threadIdx.x];
+      wb = sidx[T + threadIdx.x];
+    }
     if (!special) {
-      const double2 wb = cmul(omegaN(a.thi, a.tlo, a.ts, a.tmask, kA), wt);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {  // bin k2 of column kA <-> bin H-1-k2 of column kB
         const int k2 = threadIdx.x + j * T;
@@ -410,7 +425,6 @@ __device__ __forceinline__ void tall_body(const TallArgs &a, int blk, S sync = S
           if (p != i) sm[pad(p)] = zb;
         }
       }
-      const double2 wb = cmul(omegaN(a.thi, a.tlo, a.ts, a.tmask, W / 2), wt);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {  // column W/2: k2 <-> H-1-k2
         const int i = threadIdx.x + j * T;
@@ -536,10 +550,35 @@ __device__ __forceinline__ void fall_stages(const double2 *tw, int t, S sync, LD
 // Shared memory of a tall_any CTA (double2 entries): 2*PP padded columns,
 // the stage twiddles, and per column the factors w_N^(k1*M0*r) of the first
 // stage's loads (r < a[0], M0 = H/a[0]) and w_N^(k1*NS*r) of the last
-// stage's stores (r < a[N-1], NS = H/a[N-1]).
+// stage's stores (r < a[N-1], NS = H/a[N-1]); where that leaves as many CTAs
+// on an SM, also the H-point table of the pairing and each thread's column
+// twiddles w_N^(k1*j).
 template <class P, int PP>
-__host__ __device__ constexpr int tall_any_smem() {
+__host__ __device__ constexpr int tall_any_base() {
   return 2 * PP * col_slots<P::L>() + tw_size<P>() + 2 * PP * (P::a[0] + P::a[P::N - 1]);
+}
+template <class P, int TC>
+__host__ __device__ constexpr int tall_any_nb() {  // butterflies per thread of the first or last stage
+  constexpr int m0 = P::L / P::a[0], mn = P::L / P::a[P::N - 1];
+  return ((m0 > mn ? m0 : mn) + TC - 1) / TC;
+}
+template <class P, int TC, int PP>
+__host__ __device__ constexpr int tall_any_more() {
+  return P::L + 2 * PP * TC * tall_any_nb<P, TC>();
+}
+__host__ __device__ constexpr int ctas_per_sm(int entries, int threads) {
+  const int mem = 227 * 1024 / (16 * entries + 1024), reg = 65536 / (128 * ((threads + 31) / 32 * 32));
+  const int m = reg < 1 ? 1 : reg;
+  return mem < m ? mem : m;
+}
+template <class P, int TC, int PP>
+__host__ __device__ constexpr bool tall_any_tables() {
+  constexpr int b = tall_any_base<P, PP>(), m = tall_any_more<P, TC, PP>(), t = 2 * PP * TC;
+  return ctas_per_sm(b + m, t) >= ctas_per_sm(b, t);
+}
+template <class P, int TC, int PP>
+__host__ __device__ constexpr int tall_any_smem() {
+  return tall_any_base<P, PP>() + (tall_any_tables<P, TC, PP>() ? tall_any_more<P, TC, PP>() : 0);
 }
 
 template <class P, int TC, int PP, class S = CtaSync>
@@ -549,6 +588,10 @@ __device__ __forceinline__ void tall_any_body(const TallArgs &a, int blk, S sync
   extern __shared__ double2 sm[];
   double2 *stw = sm + 2 * PP * CS;
   double2 *fac = stw + tw_size<P>();
+  constexpr bool kTables = tall_any_tables<P, TC, PP>();
+  constexpr int NB = tall_any_nb<P, TC>(), MX = M0 > NSN ? M0 : NSN;
+  double2 *th = fac + 2 * PP * FS;            // w_H^k
+  double2 *sb = th + H + threadIdx.x;         // w_N^(k1*j) of butterfly j = t + b*TC at sb[b*T]
   const int units = a.W / 2;
   const int col = threadIdx.x / TC, t = threadIdx.x - col * TC;  // col < 2*PP
   const int pl = col >> 1;
@@ -566,6 +609,20 @@ __device__ __forceinline__ void tall_any_body(const TallArgs &a, int blk, S sync
     const int cp = blk * PP + (cc >> 1);
     const int kk = cp >= units ? 0 : (cc & 1) ? (cp == 0 ? W / 2 : W - cp) : cp;
     fac[i] = omegaN(a.thi, a.tlo, a.ts, a.tmask, r < R0 ? kk * M0 * r : kk * NSN * (r - R0));
+  }
+  // the table loads of the column twiddles and of the pairing come before the
+  // wait for the previous pass: in the passes of a few microseconds that most
+  // of these lengths run, their latency was a third of the time (160K: 2.6 K
+  // of 8.7 K cycles in the pairing)
+  double2 wbk = make_double2(1.0, 0.0);  // w_N^kb of the pairing
+  if constexpr (kTables) {
+    for (int i = threadIdx.x; i < H; i += T) cp_async16(&th[i], &a.twH[i]);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const int j = t + b * TC;
+      if (MX % TC == 0 || j < MX) sb[b * T] = omegaN(a.thi, a.tlo, a.ts, a.tmask, k1 * j);
+    }
+    wbk = omegaN(a.thi, a.tlo, a.ts, a.tmask, special ? W / 2 : active ? kA : 0);
   }
   griddep_wait();
   griddep_release();
@@ -585,7 +642,7 @@ __device__ __forceinline__ void tall_any_body(const TallArgs &a, int blk, S sync
   auto ld = [&](int e, int, int) { return row[pad(e)]; };
   auto st = [&](int e, int, int, double2 v) { row[pad(e)] = v; };
   auto ld_first = [&](int e, int j, int r) {
-    if (r == 0) base = omegaN(a.thi, a.tlo, a.ts, a.tmask, k1 * j);
+    if (r == 0) base = kTables ? sb[(j - t) / TC * T] : omegaN(a.thi, a.tlo, a.ts, a.tmask, k1 * j);
     return active ? cmul(gcol[e], r == 0 ? base : cmul(base, fc[r])) : make_double2(0.0, 0.0);
   };
   fall_stages<P, 0, 1, TC, +1, false, true>(stw, t, sync, ld_first, st, ld, st);
@@ -593,11 +650,12 @@ __device__ __forceinline__ void tall_any_body(const TallArgs &a, int blk, S sync
     const int ti = threadIdx.x - 2 * pl * TC;  // thread of the pair, < 2*TC
     double2 *ra = sm + 2 * pl * CS, *rb = ra + CS;
     // pairing twiddle w_N^(kb + W*k2) = w_N^kb * w_H^k2
+    auto wh = [&](int i) { return kTables ? th[i] : __ldg(&a.twH[i]); };
+    if constexpr (!kTables) wbk = omegaN(a.thi, a.tlo, a.ts, a.tmask, special ? W / 2 : kA);
     if (!special) {
-      const double2 wb = omegaN(a.thi, a.tlo, a.ts, a.tmask, kA);
       for (int k2 = ti; k2 < H; k2 += 2 * TC) {  // bin k2 of column kA <-> bin H-1-k2 of column kB
         double2 za = ra[pad(k2)], zb = rb[pad(H - 1 - k2)];
-        pair_square(za, zb, cmul(wb, __ldg(&a.twH[k2])));
+        pair_square(za, zb, cmul(wbk, wh(k2)));
         ra[pad(k2)] = za;
         rb[pad(H - 1 - k2)] = zb;
       }
@@ -605,14 +663,13 @@ __device__ __forceinline__ void tall_any_body(const TallArgs &a, int blk, S sync
       for (int i = ti; i <= H / 2; i += 2 * TC) {  // column 0: k2 <-> (H-k2) mod H
         const int p2 = (H - i) % H;
         double2 za = ra[pad(i)], zb = ra[pad(p2)];
-        pair_square(za, zb, __ldg(&a.twH[i]));
+        pair_square(za, zb, wh(i));
         ra[pad(i)] = za;
         if (p2 != i) ra[pad(p2)] = zb;
       }
-      const double2 wb = omegaN(a.thi, a.tlo, a.ts, a.tmask, W / 2);
       for (int i = ti; i < H / 2; i += 2 * TC) {  // column W/2: k2 <-> H-1-k2
         double2 za = rb[pad(i)], zb = rb[pad(H - 1 - i)];
-        pair_square(za, zb, cmul(wb, __ldg(&a.twH[i])));
+        pair_square(za, zb, cmul(wbk, wh(i)));
         rb[pad(i)] = za;
         rb[pad(H - 1 - i)] = zb;
       }
@@ -620,7 +677,7 @@ __device__ __forceinline__ void tall_any_body(const TallArgs &a, int blk, S sync
   }
   sync();
   auto st_last = [&](int e, int j, int r, double2 v) {
-    if (r == 0) base = omegaN(a.thi, a.tlo, a.ts, a.tmask, k1 * j);
+    if (r == 0) base = kTables ? sb[(j - t) / TC * T] : omegaN(a.thi, a.tlo, a.ts, a.tmask, k1 * j);
     if (active) gcol[e] = cmulc(v, r == 0 ? base : cmul(base, fc[R0 + r]));
   };
   fall_stages<P, 0, 1, TC, -1, true, false>(stw, t, sync, ld, st_last, ld, st);
