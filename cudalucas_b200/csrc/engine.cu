@@ -972,6 +972,7 @@ struct ll_ctx {
   bool started = false;
   int inject = 0;
   bool pdl = false;  // chain the passes with programmatic dependent launch
+  int carveout = -1;  // shared-memory part of the L1 that both passes ask for, percent
   const FusedKernel *fused = nullptr;  // iterations as one cooperative launch
   int fused_grid = 0;
   const ClusterKernel *cluster = nullptr;  // iterations as one cluster-resident launch
@@ -1095,6 +1096,20 @@ static ll_status build_tables(ll_ctx *ctx) {
   return LL_OK;
 }
 
+// The shared-memory part of the L1 (percent of 228 KB) that the CTAs of both
+// passes need on an SM, `bw` and `bt` of them fitting at most (us per
+// iteration, the driver's choice against this: 336K 15.5 / 12.1, 512K 14.1 /
+// 11.8, 576K 26.0 / 15.7, 768K 20.4 / 18.5).  -1, the driver's choice, where
+// less than 72 KB would be left to the L1: there the early launch gains less
+// than the tables lose (720K 19.1 / 19.7, 1600K 37.2 / 39.4, 4608K 84.0 / 90.6).
+static int carveout_for(const ll_ctx *ctx, int sms, int bw, int bt) {
+  const Shape &s = ctx->shape;
+  const long long cw = std::min<long long>(bw, (s.H / s.G + sms - 1) / sms), ct = std::min<long long>(bt, (tall_grid(s) + sms - 1) / sms);
+  const long long bytes = cw * ((long long)shape_wide_smem(s) + 1024) + ct * ((long long)shape_tall_smem(s) + 1024);
+  const long long percent = (100 * bytes + 228 * 1024 - 1) / (228 * 1024);
+  return percent <= 68 ? (int)percent : -1;
+}
+
 extern "C" {
 
 const char *ll_status_string(ll_status s) {
@@ -1202,6 +1217,11 @@ ll_status ll_create(int device, uint32_t q, uint32_t n, const ll_tuning *tuning,
         const long long ww = ((long long)(s.H / s.G) + (long long)sms * bw - 1) / ((long long)sms * bw);
         const long long wt = ((long long)tall_grid(s) + (long long)sms * bt - 1) / ((long long)sms * bt);
         ctx->pdl = ww <= 4 && wt <= 4;
+        // The early launch needs an SM that holds CTAs of both passes, and
+        // kernels that run with different shared-memory parts of the L1 never
+        // share one: both ask for the same part, enough for their CTAs
+        // together, and leave the rest to the L1 (tables).
+        ctx->carveout = carveout_for(ctx, sms, bw, bt);
       }
     }
     // On request, short lengths with a fused kernel run their plain
@@ -1309,22 +1329,35 @@ ll_status ll_create(int device, uint32_t q, uint32_t n, const ll_tuning *tuning,
 
 void ll_destroy(ll_ctx *ctx) { free_ctx(ctx); }
 
+// Launch attributes of a pass: its shared-memory part of the L1 (percent, or
+// -1: the driver's choice) and programmatic stream serialization.
+static void pass_attributes(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr, bool chained, int carveout) {
+  unsigned n = 0;
+  if (carveout >= 0) {
+    attr[n].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[n++].val.sharedMemCarveout = (unsigned)carveout;
+  }
+  if (chained) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+}
+
 // Launches a specialised pass.  `chained`: the previous operation in the
 // stream is the other pass, so the launch may use programmatic stream
 // serialization (the kernel runs its prologue while that pass drains and
 // waits in griddep_wait() before touching the state).
 static void launch_static(const void *k, void *args, int grid, int threads, size_t smem, cudaStream_t st,
-                          bool chained) {
+                          bool chained, int carveout) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = chained ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  pass_attributes(cfg, attr, chained, carveout);
   void *argv[] = {args};
   cudaLaunchKernelExC(&cfg, k, argv);
 }
@@ -1334,7 +1367,7 @@ static void launch_wide(ll_ctx *ctx, int mode, bool chained = false) {
   const size_t sm = shape_wide_smem(s);
   if (s.sw) {
     void (*k)(WideArgs) = mode == WIDE_INIT ? s.sw->init : mode == WIDE_REPORT ? s.sw->report : s.sw->iter;
-    launch_static((const void *)k, &ctx->wa, s.H / s.G, s.T1, sm, ctx->stream, chained && ctx->pdl);
+    launch_static((const void *)k, &ctx->wa, s.H / s.G, s.T1, sm, ctx->stream, chained && ctx->pdl, ctx->carveout);
   } else if (mode == WIDE_INIT) {
     wide_kernel<EPT, WIDE_INIT><<<s.H / s.G, s.T1, sm, ctx->stream>>>(ctx->wa);
   } else if (mode == WIDE_REPORT) {
@@ -1346,7 +1379,7 @@ static void launch_wide(ll_ctx *ctx, int mode, bool chained = false) {
 
 static void launch_tall(ll_ctx *ctx, bool chained = false) {
   const Shape &s = ctx->shape;
-  if (s.st) launch_static((const void *)s.st->run, &ctx->ta, tall_grid(s), s.T2, shape_tall_smem(s), ctx->stream, chained && ctx->pdl);
+  if (s.st) launch_static((const void *)s.st->run, &ctx->ta, tall_grid(s), s.T2, shape_tall_smem(s), ctx->stream, chained && ctx->pdl, ctx->carveout);
   else tall_kernel<EPT><<<s.W / 2, s.T2, tall_smem(s.H), ctx->stream>>>(ctx->ta);
 }
 
