@@ -387,7 +387,8 @@ struct StaticWide {
   int extra;  // shared-memory entries beyond the rows (stage twiddles)
   int rows;   // shared-memory entries of the G rows
   int tr;     // threads per row (a thread's elements are t + r*tr)
-  int alt;    // 1: the alternative row kernel of its length (LL_KERNELS_ALT_WIDE)
+  int alt;    // kAltRows: the alternative row kernel of its length (LL_KERNELS_ALT_WIDE);
+              // kShortRows: the one for passes of few row groups
 };
 struct StaticTall {
   int L;
@@ -400,6 +401,7 @@ struct StaticTall {
   int ppc;      // column pairs per CTA
 };
 
+enum { kAltRows = 1, kShortRows = 2 };
 #define LLB_WIDE(LIST, G)                                                                                       \
   {LIST::L, G, wide_static<LIST, G, WIDE_ITER>, wide_static<LIST, G, WIDE_REPORT>, wide_static<LIST, G, WIDE_INIT>, \
    wide_static_batch<LIST, G>,                                                                                  \
@@ -407,12 +409,12 @@ struct StaticTall {
    G * row_slots<LIST::L, G>(), LIST::L / 16, 0}
 // rows through shared memory with few elements per thread (wide_any); MINB
 // CTAs per SM asked of the register allocator
-#define LLB_WIDE_ANY(LIST, G, MINB)                                                                         \
+#define LLB_WIDE_ANY(LIST, G, MINB, KIND)                                                                        \
   {LIST::L, G, wide_any<LIST, G, MINB, WIDE_ITER>, wide_any<LIST, G, MINB, WIDE_REPORT>,                     \
    wide_any<LIST, G, MINB, WIDE_INIT>, wide_any_batch<LIST, G, MINB>,                                        \
    LIST::N, {LIST::a[0], LIST::N > 1 ? LIST::a[1 % LIST::N] : 0, LIST::N > 2 ? LIST::a[2 % LIST::N] : 0,       \
              LIST::N > 3 ? LIST::a[3 % LIST::N] : 0},                                                          \
-   tw_size<LIST>(), G * row_slots<LIST::L, G>(), LIST::L / LIST::a[0], 1}
+   tw_size<LIST>(), G * row_slots<LIST::L, G>(), LIST::L / LIST::a[0], KIND}
 #define LLB_RAD(LIST)                                                                                 \
   LIST::N, {LIST::a[0], LIST::N > 1 ? LIST::a[1 % LIST::N] : 0, LIST::N > 2 ? LIST::a[2 % LIST::N] : 0, \
             LIST::N > 3 ? LIST::a[3 % LIST::N] : 0}
@@ -497,29 +499,43 @@ using C4000 = RList<10, 10, 10, 4>;
 using C4050 = RList<5, 9, 9, 10>;
 using C4374 = RList<9, 9, 9, 6>;
 
-// Alternative row kernels (opt-in, LL_KERNELS_ALT_WIDE): twice the warps per
-// SM (64-80 registers, 3 CTAs of 8 or 10 warps) but every stage through
-// shared memory.  Measured (ms/iter, alternative against default): 2048K
-// 0.0435 / 0.0366, 3200K 0.0679 / 0.0629, 3136K 0.0643 / 0.0650, 1440K
-// 0.0382 / 0.0418.
-// Rows of 2048 (8x4x8x8) and 3072 (8x6x8x8) measured slower too: 12288K
-// 0.2730 / 0.2560, 18432K 0.4102 / 0.3775; they are not compiled.
-using A1280 = RList<8, 4, 5, 8>;  // 160 threads per row, 8 elements each
-using A1024 = RList<8, 4, 4, 8>;
+// Rows with few elements per thread (wide_any): every stage in shared memory,
+// but shorter carry phases, which are most of a short pass, and twice to four
+// times the warps.  At 256 and 512 they replace the 16-element kernels for
+// passes of at most kShortGroups row groups (us per iteration, 16 elements
+// against few): 50K 9.3 / 6.7, 160K 10.8 / 8.7, 192K 12.1 / 9.8, 384K (256 x
+// 768) 13.2 / 11.9, 512K 13.3 / 11.8, 800K 25.6 / 19.8, but 256 x 1024 13.6 /
+// 14.7, 512 x 1024 18.7 / 25.1.  At 768 and above they gain in places only
+// (336K 15.5 / 12.1, 864K 24.6 / 21.2; 1152K 29.3 / 31.5) and are opt-in
+// (LL_KERNELS_ALT_WIDE, and the launch preferences below).  Rows of 1536 and
+// 1792 measured slower throughout (1728K 32.3 / 37.9, 6272K 117 / 139), rows
+// of 2048 and 3072 too; they are not compiled.
+using F256 = RList<4, 4, 4, 4>;   // 64 threads per row, 4 elements each
+using F512 = RList<8, 8, 8>;      // 64 threads per row, 8 elements each
+using F768 = RList<8, 12, 8>;     // 96
+using F1024 = RList<8, 16, 8>;    // 128
+using F1280 = RList<8, 4, 5, 8>;  // 160
+constexpr int kShortGroups = 400;
 static const StaticWide kWide[] = {
     LLB_WIDE(L256, 4),  LLB_WIDE(L256, 2),  LLB_WIDE(L512, 4),  LLB_WIDE(L768, 4),  LLB_WIDE(L1024, 2), LLB_WIDE(L1280, 2),
     LLB_WIDE(L1536, 2), LLB_WIDE(L1792, 2), LLB_WIDE(L2048, 2), LLB_WIDE(L2304, 2),
     LLB_WIDE(L2560, 2), LLB_WIDE(L3072, 2), LLB_WIDE(L3584, 1), LLB_WIDE(L4096, 1),
-    LLB_WIDE_ANY(A1280, 2, 3), LLB_WIDE_ANY(A1024, 2, 3),
+    LLB_WIDE_ANY(F256, 2, 4, kShortRows), LLB_WIDE_ANY(F512, 2, 4, kShortRows), LLB_WIDE_ANY(F768, 2, 2, kAltRows),
+    LLB_WIDE_ANY(F1024, 2, 2, kAltRows), LLB_WIDE_ANY(F1280, 2, 3, kAltRows),
 };
-// the row kernel variants a context may use: with LL_KERNELS_ALT_WIDE the
-// alternative kernel of a length replaces the others of that length
-static bool wide_allowed(const StaticWide &w, const ll_tuning *t) {
+// The row kernel variants a context of N = L*H may use: with
+// LL_KERNELS_ALT_WIDE the alternative kernel of a length replaces the others
+// of that length; for few row groups the short one does (not with
+// LL_KERNELS_FUSED, whose kernels are those of 16 elements per thread).
+static bool short_rows(const StaticWide &k, long long N, const ll_tuning *t) {
+  return k.alt == kShortRows && N / k.L / k.G <= kShortGroups && !(t && (t->kernels & LL_KERNELS_FUSED));
+}
+static bool wide_allowed(const StaticWide &w, long long N, const ll_tuning *t) {
   const bool want_alt = t && (t->kernels & LL_KERNELS_ALT_WIDE);
+  if (w.alt == kShortRows) return short_rows(w, N, t);
   if (w.alt) return want_alt;
-  if (!want_alt) return true;
   for (const auto &k : kWide)
-    if (k.alt && k.L == w.L) return false;
+    if (k.L == w.L && ((k.alt == kAltRows && want_alt) || short_rows(k, N, t))) return false;
   return true;
 }
 // Column lengths outside the 16 x M x 16 family that the length policy meets
@@ -769,7 +785,7 @@ bool choose_shape(long long N, const ll_tuning *t, Shape &out) {
     const StaticTall *bt = nullptr;
     double best = 1e30;
     for (const auto &w : kWide) {
-      if (N % w.L || !wide_allowed(w, t)) continue;
+      if (N % w.L || !wide_allowed(w, N, t)) continue;
       if (t && t->width > 0 && t->width != w.L) continue;
       const long long H = N / w.L;
       const StaticTall *tt = find_tall((int)H);
@@ -794,7 +810,7 @@ bool choose_shape(long long N, const ll_tuning *t, Shape &out) {
     // a specialised wide pass with the generic tall pass, when the columns
     // have no specialised length (the wide pass is the costlier one)
     for (const auto &w : kWide) {
-      if (N % w.L || !wide_allowed(w, t)) continue;
+      if (N % w.L || !wide_allowed(w, N, t)) continue;
       if (t && t->width > 0 && t->width != w.L) continue;
       const long long H = N / w.L;
       Shape s;
