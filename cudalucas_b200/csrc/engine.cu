@@ -34,6 +34,7 @@
 // while the previous pass drains, and wait (griddepcontrol.wait) before they
 // touch the state.
 #include <cooperative_groups.h>
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stddef.h>
@@ -63,12 +64,24 @@ struct DevState {
   uint32_t fault;             // bit 0: wait timeout, bit 1: carry overflow
   uint32_t bar_count;         // grid barrier of the fused kernel: arrivals
   uint32_t bar_gen;           //   and generation
-  uint32_t pad_;
+  uint32_t pipe_ticket;       // persistent row pass: tickets drawn in this launch
+  uint32_t pipe_exit;         //   and CTAs that have left
+  uint32_t pad_[3];
 };
+
+// Constants of a row m2 (its words 2*m2 and 2*m2+1): exponents rowE, weights
+// rowW and rowWi; a multiple of 16 bytes for the copy engine.
+struct RowConst {
+  int32_t e0, e1;
+  double w0, w1, wi0, wi1;
+  double pad_;
+};
+using TileMap = CUtensorMap;  // of the state array: boxes of two rows m2, 256 columns k1
 
 struct TallArgs {
   double2 *A;
   const double2 *stw;   // stage twiddles of the specialised column transform
+  const double2 *ptw;   // twiddles of the persistent column pass (kernels_pipe.cuh)
   const double2 *twH;   // e^{2 pi i e/H}
   const double2 *thi;   // e^{2 pi i (e<<TS)/N}
   const double2 *tlo;   // e^{2 pi i e/N}, e < 2^TS
@@ -82,9 +95,11 @@ struct TallArgs {
 struct WideArgs {
   double2 *A;
   const double2 *stw;   // stage twiddles of the specialised row transform
+  const double2 *ptw;   // twiddles of the persistent row pass (kernels_pipe.cuh)
+  const RowConst *rowC; // rowE, rowW, rowWi by row
   int32_t *xint;
   long long *carry;     // carries, one row of W per CTA: packed pairs (generic) or doubles
-  uint32_t *flags;      // ready flags of the generic kernels, one per CTA
+  uint32_t *flags;      // ready flags: of the generic kernels' CTAs, or of the persistent pass's extra tickets
   const double2 *twW;
   const int32_t *rowE;  // ((-(2*m2+t)*b) mod n), 2H entries
   const double *rowW;   // 2^(rowE/n)
@@ -95,6 +110,7 @@ struct WideArgs {
   DevState *st;
   FftPlan pw;
   int W, H, G, ngroups;
+  int chains, chain_len;  // persistent row pass: runs of units that advance side by side
   int pf;  // > 0: prefetch into L2 the row group pf tickets ahead (state larger than L2)
   uint32_t q, n, b, qn;
   double inv_q, inv_n, inv_H;  // reciprocals for udiv_est
@@ -374,6 +390,7 @@ __global__ void __launch_bounds__(256) wide_kernel(WideArgs a) {
 }
 
 #include "kernels_static.cuh"
+#include "kernels_pipe.cuh"
 #include "kernels_cluster.cuh"
 
 // Registry of compile-time specialised kernels, by row length.
@@ -520,15 +537,16 @@ static const StaticWide kWide[] = {
     LLB_WIDE(L256, 4),  LLB_WIDE(L256, 2),  LLB_WIDE(L512, 4),  LLB_WIDE(L768, 4),  LLB_WIDE(L1024, 2), LLB_WIDE(L1280, 2),
     LLB_WIDE(L1536, 2), LLB_WIDE(L1792, 2), LLB_WIDE(L2048, 2), LLB_WIDE(L2304, 2),
     LLB_WIDE(L2560, 2), LLB_WIDE(L3072, 2), LLB_WIDE(L3584, 1), LLB_WIDE(L4096, 1),
-    LLB_WIDE_ANY(F256, 2, 4, kShortRows), LLB_WIDE_ANY(F512, 2, 4, kShortRows), LLB_WIDE_ANY(F768, 2, 2, kAltRows),
+    LLB_WIDE_ANY(F256, 2, 4, kShortRows), LLB_WIDE_ANY(F512, 2, 4, kShortRows), LLB_WIDE_ANY(F512, 4, 2, kAltRows),
+    LLB_WIDE_ANY(F768, 2, 2, kAltRows),
     LLB_WIDE_ANY(F1024, 2, 2, kAltRows), LLB_WIDE_ANY(F1280, 2, 3, kAltRows),
 };
 // The row kernel variants a context of N = L*H may use: with
 // LL_KERNELS_ALT_WIDE the alternative kernel of a length replaces the others
-// of that length; for few row groups the short one does (not with
-// LL_KERNELS_FUSED, whose kernels are those of 16 elements per thread).
+// of that length; for few row groups the short one does, unless the caller
+// chooses kernels (then 16 elements per thread, as the fused kernels have).
 static bool short_rows(const StaticWide &k, long long N, const ll_tuning *t) {
-  return k.alt == kShortRows && N / k.L / k.G <= kShortGroups && !(t && (t->kernels & LL_KERNELS_FUSED));
+  return k.alt == kShortRows && N / k.L / k.G <= kShortGroups && !(t && t->kernels);
 }
 static bool wide_allowed(const StaticWide &w, long long N, const ll_tuning *t) {
   const bool want_alt = t && (t->kernels & LL_KERNELS_ALT_WIDE);
@@ -609,6 +627,40 @@ static const FusedKernel kFused[] = {
 static const FusedKernel *find_fused(int W, int H, int G) {
   for (const auto &k : kFused)
     if (k.W == W && k.H == H && k.G == G) return &k;
+  return nullptr;
+}
+
+// Persistent passes (kernels_pipe.cuh), by row or column length 256*M.
+struct PipeKernel {
+  int L;
+  void (*wide)(TileMap, WideArgs);
+  void (*tall)(TallArgs);
+  int threads, tw, slots, smem_wide, smem_tall;
+};
+#define LLB_PIPE(M) \
+  {256 * M, wide_pipe<M>, tall_pipe<M>, Pipe<M>::NT, Pipe<M>::TWN, Pipe<M>::NS, wide_pipe_smem<M>(), tall_pipe_smem<M>()}
+static const PipeKernel kPipe[] = {
+    {1024, wide_pipe<4>, nullptr, Pipe<4>::NT, Pipe<4>::TWN, Pipe<4>::NS, wide_pipe_smem<4>(), 0},
+    LLB_PIPE(5), LLB_PIPE(6),  LLB_PIPE(7),  LLB_PIPE(8),  LLB_PIPE(9),
+    LLB_PIPE(10), LLB_PIPE(12), LLB_PIPE(14), LLB_PIPE(16),
+};
+// Where the persistent passes are used (us per iteration, launch per unit
+// against persistent).  They lose while an SM has few units, since their CTAs
+// start with one load per SM and share it between few groups: rows, 2048K
+// (1024 x 1024) 35.0 / 42.2, 2880K (2560 x 576) 56.8 / 61.9, but 3024K (2304 x
+// 672) 69.1 / 60.3, 3136K (1024 x 1568) 60.6 / 56.3, 3200K 66.0 / 57.4, 18432K
+// 366 / 290, 32768K 796 / 582; rows of 1792, whose groups are seven warps, gain
+// from 9000K on (6272K 116 / 118, 9408K 221 / 216, 14336K 277 / 266); rows up
+// to 768 never do (4320K 93.5 / 95.2).  Columns, 2048K (512 x 2048) 33.2 /
+// 33.8, 4096K (2048 x 1024) 67.2 / 70.0, but 2304K (512 x 2304) 40.4 / 38.1,
+// 3200K 57.4 / 55.2, 18432K 290 / 266.
+static bool pipe_rows(long long W, long long n) {
+  return W >= 1024 && n >= 3000 * 1024 && (W != 1792 || n >= 9000 * 1024);
+}
+static bool pipe_columns(long long H, long long n) { return H >= 1280 && n >= 2304 * 1024; }
+static const PipeKernel *find_pipe(int L) {
+  for (const auto &k : kPipe)
+    if (k.L == L) return &k;
   return nullptr;
 }
 
@@ -889,6 +941,22 @@ std::vector<double2> stage_twiddles(const int *rad, int nrad) {
 
 }  // namespace
 
+// Twiddle table of the persistent passes for length L = 256*M (see
+// kernels_pipe.cuh): entry e < 8 of thread c at [e*TR + c], then the stage-1
+// twiddles w_TR^(j0*v) at rows of odd stride.
+static std::vector<double2> pipe_twiddles(int L) {
+  const int M = L / 256, TR = L / 16, SS = M | 1;
+  std::vector<double2> out((size_t)8 * TR + (M > 1 ? 16 * SS : 0), make_double2(0.0, 0.0));
+  static const int power[8] = {8, 4, 2, 2, 1, 1, 1, 1}, root[8] = {0, 0, 0, 2, 0, 1, 2, 3};
+  for (int c = 0; c < TR; ++c)
+    for (int e = 0; e < 8; ++e)
+      out[(size_t)e * TR + c] = unit_root((unsigned long long)power[e] * c + (unsigned long long)root[e] * (L / 16), L);
+  if (M > 1)
+    for (int j = 0; j < 16; ++j)
+      for (int v = 0; v < M; ++v) out[(size_t)8 * TR + j * SS + v] = unit_root((unsigned long long)j * v, TR);
+  return out;
+}
+
 // Launch preferences measured on the B200 for lengths of the reference's
 // table where the engine's default shape (row width nearest sqrt(N)) is not
 // the fastest: the row width and ll_tuning.kernels to use when the caller
@@ -980,6 +1048,11 @@ struct ll_ctx {
   DevState *st = nullptr;
   double2 *twW = nullptr, *twH = nullptr, *thi = nullptr, *tlo = nullptr;
   double2 *stwW = nullptr, *stwH = nullptr;
+  const PipeKernel *pipe_w = nullptr, *pipe_t = nullptr;  // persistent passes of plain iterations
+  int pipe_grid_w = 0, pipe_grid_t = 0;
+  TileMap map{};
+  double2 *ptwW = nullptr, *ptwH = nullptr;
+  RowConst *rowC = nullptr;
   int32_t *rowE = nullptr, *colF = nullptr;
   double *rowW = nullptr, *rowWi = nullptr, *colW = nullptr, *colWi = nullptr;
   // host mirror
@@ -1028,7 +1101,7 @@ static void free_ctx(ll_ctx *c) {
   int prev = 0;
   cudaGetDevice(&prev);
   cudaSetDevice(c->device);
-  void *ptrs[] = {c->A, c->xint, c->ck_digits, c->carry, c->flags, c->st, c->twW, c->twH, c->thi, c->tlo, c->stwW, c->stwH, c->stwC,
+  void *ptrs[] = {c->A, c->xint, c->ck_digits, c->carry, c->flags, c->st, c->twW, c->twH, c->thi, c->tlo, c->stwW, c->stwH, c->stwC, c->ptwW, c->ptwH, c->rowC,
                   c->rowE, c->colF, c->rowW, c->rowWi, c->colW, c->colWi};
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -1103,6 +1176,14 @@ static ll_status build_tables(ll_ctx *ctx) {
     if ((int)t.size() != ctx->shape.st->tw) return LL_ERR_SHAPE;
     CK(upload(&ctx->stwH, t));
   }
+  if (ctx->pipe_w) {
+    CK(upload(&ctx->ptwW, pipe_twiddles(W)));
+    std::vector<RowConst> rc(H);
+    for (int m2 = 0; m2 < H; ++m2)
+      rc[m2] = {rE[2 * m2], rE[2 * m2 + 1], rW[2 * m2], rW[2 * m2 + 1], rWi[2 * m2], rWi[2 * m2 + 1], 0.0};
+    CK(upload(&ctx->rowC, rc));
+  }
+  if (ctx->pipe_t) CK(upload(&ctx->ptwH, pipe_twiddles(H)));
   CK(upload(&ctx->rowE, rE));
   CK(upload(&ctx->rowW, rW));
   CK(upload(&ctx->rowWi, rWi));
@@ -1120,10 +1201,52 @@ static ll_status build_tables(ll_ctx *ctx) {
 // than the tables lose (720K 19.1 / 19.7, 1600K 37.2 / 39.4, 4608K 84.0 / 90.6).
 static int carveout_for(const ll_ctx *ctx, int sms, int bw, int bt) {
   const Shape &s = ctx->shape;
+  if (ctx->pipe_w || ctx->pipe_t) return -1;
   const long long cw = std::min<long long>(bw, (s.H / s.G + sms - 1) / sms), ct = std::min<long long>(bt, (tall_grid(s) + sms - 1) / sms);
   const long long bytes = cw * ((long long)shape_wide_smem(s) + 1024) + ct * ((long long)shape_tall_smem(s) + 1024);
   const long long percent = (100 * bytes + 228 * 1024 - 1) / (228 * 1024);
   return percent <= 68 ? (int)percent : -1;
+}
+
+// Whether the plain iterations of a context run the persistent passes.
+static void choose_pipe(ll_ctx *ctx, const ll_tuning *tuning) {
+  const Shape &s = ctx->shape;
+  int sms = 0;
+  if (!s.sw || !s.st || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess)
+    return;
+  const PipeKernel *w = s.H % 2 == 0 && s.sw->tr == s.W / 16 && pipe_rows(s.W, ctx->n) ? find_pipe(s.W) : nullptr;
+  const PipeKernel *t = pipe_columns(s.H, ctx->n) ? find_pipe(s.H) : nullptr;
+  if (w && cudaFuncSetAttribute(w->wide, cudaFuncAttributeMaxDynamicSharedMemorySize, w->smem_wide) == cudaSuccess) {
+    ctx->pipe_w = w;
+    ctx->pipe_grid_w = std::min(sms, s.H / 2);
+  }
+  if (t && t->tall && cudaFuncSetAttribute(t->tall, cudaFuncAttributeMaxDynamicSharedMemorySize, t->smem_tall) == cudaSuccess) {
+    ctx->pipe_t = t;
+    ctx->pipe_grid_t = std::min(sms, s.W / 2);
+  }
+  cudaGetLastError();
+}
+
+// The tensor map of the state array for the persistent row pass: W lines of
+// 2*H doubles, boxes of two rows m2 (32 bytes) by 256 columns k1.
+static ll_status encode_map(ll_ctx *ctx) {
+  using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                              const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                              CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  void *fn = nullptr;
+  cudaDriverEntryPointQueryResult found;
+  CK(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found));
+  const cuuint64_t dims[2] = {2 * (cuuint64_t)ctx->shape.H, (cuuint64_t)ctx->shape.W};
+  const cuuint64_t strides[1] = {16 * (cuuint64_t)ctx->shape.H};
+  const cuuint32_t box[2] = {4, 256}, step[2] = {1, 1};
+  if (!fn || found != cudaDriverEntryPointSuccess ||
+      ((Encode)fn)(&ctx->map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, ctx->A, dims, strides, box, step,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+    ctx->err = "cuTensorMapEncodeTiled";
+    return LL_ERR_CUDA;
+  }
+  return LL_OK;
 }
 
 extern "C" {
@@ -1172,20 +1295,26 @@ ll_status ll_create(int device, uint32_t q, uint32_t n, const ll_tuning *tuning,
     e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) { rc = cuda_fail(ctx, e, "stream"); break; }
     const int ngroups = s.H / s.G;
+    choose_pipe(ctx, tuning);
+    const size_t flag_bytes = sizeof(uint32_t) * (size_t)std::max(ngroups, 64);
+    // a row of carries per row group, or per unit of two rows of the
+    // persistent pass
+    const size_t carry_bytes = sizeof(long long) * (size_t)std::max(ngroups, ctx->pipe_w ? s.H / 2 : 0) * s.W;
     if ((e = cudaMalloc((void **)&ctx->A, sizeof(double2) * (size_t)ctx->N)) != cudaSuccess ||
         (e = cudaMalloc((void **)&ctx->xint, sizeof(int32_t) * (size_t)n)) != cudaSuccess ||
-        (e = cudaMalloc((void **)&ctx->carry, sizeof(long long) * (size_t)ngroups * s.W)) != cudaSuccess ||
-        (e = cudaMalloc((void **)&ctx->flags, sizeof(uint32_t) * (size_t)ngroups)) != cudaSuccess ||
+        (e = cudaMalloc((void **)&ctx->carry, carry_bytes)) != cudaSuccess ||
+        (e = cudaMalloc((void **)&ctx->flags, flag_bytes)) != cudaSuccess ||
         (e = cudaMalloc((void **)&ctx->st, sizeof(DevState))) != cudaSuccess) {
       rc = e == cudaErrorMemoryAllocation ? LL_ERR_NOMEM : cuda_fail(ctx, e, "cudaMalloc");
       break;
     }
-    if ((e = cudaMemset(ctx->flags, 0, sizeof(uint32_t) * (size_t)ngroups)) != cudaSuccess ||
-        (s.sw && (e = cudaMemset(ctx->carry, kNoCarryByte, sizeof(long long) * (size_t)ngroups * s.W)) != cudaSuccess) ||
+    if ((e = cudaMemset(ctx->flags, 0, flag_bytes)) != cudaSuccess ||
+        (s.sw && (e = cudaMemset(ctx->carry, kNoCarryByte, carry_bytes)) != cudaSuccess) ||
         (e = cudaMemset(ctx->st, 0, sizeof(DevState))) != cudaSuccess) {
       rc = cuda_fail(ctx, e, "cudaMemset");
       break;
     }
+    if (ctx->pipe_w && (rc = encode_map(ctx)) != LL_OK) break;
     rc = build_tables(ctx);
     if (rc != LL_OK) break;
     // The dynamic shared-memory limit is a per-function (not per-context)
@@ -1309,9 +1438,16 @@ ll_status ll_create(int device, uint32_t q, uint32_t n, const ll_tuning *tuning,
       }
     }
     TallArgs &ta = ctx->ta;
-    ta.A = ctx->A; ta.stw = ctx->stwH; ta.twH = ctx->twH; ta.thi = ctx->thi; ta.tlo = ctx->tlo; ta.st = ctx->st;
+    ta.A = ctx->A; ta.ptw = ctx->ptwH; ta.stw = ctx->stwH; ta.twH = ctx->twH; ta.thi = ctx->thi; ta.tlo = ctx->tlo; ta.st = ctx->st;
     ta.ph = ctx->ph; ta.W = s.W; ta.H = s.H; ta.N = ctx->N; ta.ts = ctx->ts; ta.tmask = (1 << ctx->ts) - 1; ta.q = q;
     WideArgs &wa = ctx->wa;
+    if (ctx->pipe_w) {
+      // a multiple of the slots, about 32, of four units or more each
+      const int ns = ctx->pipe_w->slots, units = s.H / 2;
+      wa.chains = ns * std::max(1, std::min(32 / ns, units / (4 * ns)));
+      wa.chain_len = (units + wa.chains - 1) / wa.chains;
+    }
+    wa.ptw = ctx->ptwW; wa.rowC = ctx->rowC;
     wa.A = ctx->A; wa.stw = ctx->stwW; wa.xint = ctx->xint; wa.carry = ctx->carry; wa.flags = ctx->flags; wa.twW = ctx->twW;
     wa.rowE = ctx->rowE; wa.rowW = ctx->rowW; wa.rowWi = ctx->rowWi;
     wa.colF = ctx->colF; wa.colW = ctx->colW; wa.colWi = ctx->colWi;
@@ -1366,7 +1502,7 @@ static void pass_attributes(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr, 
 // serialization (the kernel runs its prologue while that pass drains and
 // waits in griddep_wait() before touching the state).
 static void launch_static(const void *k, void *args, int grid, int threads, size_t smem, cudaStream_t st,
-                          bool chained, int carveout) {
+                          bool chained, int carveout, void *args0 = nullptr) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
@@ -1374,14 +1510,18 @@ static void launch_static(const void *k, void *args, int grid, int threads, size
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   pass_attributes(cfg, attr, chained, carveout);
-  void *argv[] = {args};
+  void *argv[] = {args0 ? args0 : args, args};
   cudaLaunchKernelExC(&cfg, k, argv);
 }
 
 static void launch_wide(ll_ctx *ctx, int mode, bool chained = false) {
   const Shape &s = ctx->shape;
   const size_t sm = shape_wide_smem(s);
-  if (s.sw) {
+  if (ctx->pipe_w && mode == WIDE_ITER) {
+    const PipeKernel *p = ctx->pipe_w;
+    launch_static((const void *)p->wide, &ctx->wa, ctx->pipe_grid_w, p->threads, p->smem_wide, ctx->stream, chained,
+                  ctx->carveout, &ctx->map);
+  } else if (s.sw) {
     void (*k)(WideArgs) = mode == WIDE_INIT ? s.sw->init : mode == WIDE_REPORT ? s.sw->report : s.sw->iter;
     launch_static((const void *)k, &ctx->wa, s.H / s.G, s.T1, sm, ctx->stream, chained && ctx->pdl, ctx->carveout);
   } else if (mode == WIDE_INIT) {
@@ -1395,7 +1535,10 @@ static void launch_wide(ll_ctx *ctx, int mode, bool chained = false) {
 
 static void launch_tall(ll_ctx *ctx, bool chained = false) {
   const Shape &s = ctx->shape;
-  if (s.st) launch_static((const void *)s.st->run, &ctx->ta, tall_grid(s), s.T2, shape_tall_smem(s), ctx->stream, chained && ctx->pdl, ctx->carveout);
+  if (ctx->pipe_t) {
+    const PipeKernel *p = ctx->pipe_t;
+    launch_static((const void *)p->tall, &ctx->ta, ctx->pipe_grid_t, p->threads, p->smem_tall, ctx->stream, chained, ctx->carveout);
+  } else if (s.st) launch_static((const void *)s.st->run, &ctx->ta, tall_grid(s), s.T2, shape_tall_smem(s), ctx->stream, chained && ctx->pdl, ctx->carveout);
   else tall_kernel<EPT><<<s.W / 2, s.T2, tall_smem(s.H), ctx->stream>>>(ctx->ta);
 }
 
@@ -1619,6 +1762,13 @@ uint64_t ll_context_bytes(uint32_t q, uint32_t n, const ll_tuning *tuning) {
   b += 20 * 2 * H + 20 * W;                                                           // weights
   if (s.sw) b += 16 * (uint64_t)s.sw->extra;
   if (s.st) b += 16 * (uint64_t)s.st->tw;
+  // the persistent passes' twiddles, row constants and carry rows
+  if (s.sw && s.st) {
+    const PipeKernel *pw = H % 2 == 0 && s.sw->tr == s.W / 16 && pipe_rows(s.W, n) ? find_pipe(s.W) : nullptr;
+    const PipeKernel *pt = pipe_columns(s.H, n) ? find_pipe(s.H) : nullptr;
+    if (pw) b += 16 * (uint64_t)pw->tw + sizeof(RowConst) * H + (H / 2 > ng ? 8 * (H / 2 - ng) * W : 0);
+    if (pt && pt->tall) b += 16 * (uint64_t)pt->tw;
+  }
   // the cluster kernel's stage twiddles, when the length has one (the
   // largest table among its variants)
   uint64_t tw_cluster = 0;
@@ -1693,6 +1843,8 @@ int32_t ll_check_tables(void) {
     if ((int)stage_twiddles(k.rad, k.nrad).size() != k.extra) ++bad;
   for (const auto &k : kTall)
     if ((int)stage_twiddles(k.rad, k.nrad).size() != k.tw) ++bad;
+  for (const auto &k : kPipe)
+    if ((int)pipe_twiddles(k.L).size() != k.tw) ++bad;
   for (const auto &k : kCluster) {
     int L = 1, Lc = 1;
     for (int i = 0; i < k.nrad; ++i) L *= k.rad[i];
@@ -1793,8 +1945,10 @@ extern "C" ll_status ll_step_static(int device, uint32_t q, uint32_t n, uint32_t
   if (n > LL_STATIC_MAX_WORDS) return LL_ERR_ARG;  // beyond the static scratch's stated maximum
   if (device < 0 || device >= kMaxDevices) return LL_ERR_ARG;
   const int N = (int)(n / 2);
+  ll_tuning t{};
+  t.kernels = LL_KERNELS_NO_CLUSTER;  // the kernels of a context with two launches per iteration
   Shape s;
-  if (!choose_shape(N, nullptr, s)) return LL_ERR_SHAPE;
+  if (!choose_shape(N, &t, s)) return LL_ERR_SHAPE;
   std::lock_guard<std::mutex> lock(g_device_mu[device]);
   int prev = 0;
   cudaGetDevice(&prev);
@@ -2086,6 +2240,7 @@ static ll_status build_classes(ll_batch *b) {
   return LL_OK;
 }
 
+constexpr int kBatchCarveout = 100;
 static void launch_class(const void *kern, const void *arr, int units, int count, int threads, size_t smem,
                          cudaStream_t st, bool chained) {
   cudaLaunchConfig_t cfg = {};
@@ -2093,11 +2248,8 @@ static void launch_class(const void *kern, const void *arr, int units, int count
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = chained ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  pass_attributes(cfg, attr, chained, kBatchCarveout);
   void *argv[] = {(void *)&arr, (void *)&units};
   cudaLaunchKernelExC(&cfg, kern, argv);
 }
