@@ -967,46 +967,45 @@ struct PreferredShape {
   int32_t width;    // row width W
   int32_t kernels;  // LL_KERNELS_* flags
 };
-// (fftbench --all-shapes over the table lengths, 200 iterations timed with
-// CUDA events; kept where the preference is at least 8 % faster)
+// (every row width with specialised kernels, and the opt-in row kernels, over
+// the table lengths, 128 to 1024 iterations timed with CUDA events; kept where
+// the preference is at least 3 % faster)
 static const PreferredShape kPreferred[] = {
-    {288u * 1024, 256, 0},  // 288K: 0.0159 against 0.0220 ms/iter (W = 512)
-    {324u * 1024, 256, 0},  // 324K: 0.0176 against 0.0227 ms/iter (W = 512)
-    {336u * 1024, 768, 0},  // 336K: 0.0175 against 0.0243 ms/iter (W = 512)
-    {360u * 1024, 768, 0},  // 360K: 0.0181 against 0.0254 ms/iter (W = 512)
-    {392u * 1024, 256, 0},  // 392K: 0.0183 against 0.0255 ms/iter (W = 512)
-    {400u * 1024, 256, 0},  // 400K: 0.0184 against 0.0255 ms/iter (W = 512)
-    {448u * 1024, 1024, 0},  // 448K: 0.0181 against 0.0250 ms/iter (W = 512)
-    {576u * 1024, 1536, 0},  // 576K: 0.0212 against 0.0270 ms/iter (W = 512)
-    {640u * 1024, 256, 0},  // 640K: 0.0183 against 0.0308 ms/iter (W = 1024)
-    {672u * 1024, 1792, 0},  // 672K: 0.0232 against 0.0293 ms/iter (W = 512)
-    {768u * 1024, 256, 0},  // 768K: 0.0217 against 0.0248 ms/iter (W = 512)
-    {784u * 1024, 1792, 0},  // 784K: 0.0264 against 0.0298 ms/iter (W = 512)
-    {896u * 1024, 256, 0},  // 896K: 0.0223 against 0.0342 ms/iter (W = 1024)
-    {1024u * 1024, 512, 0},  // 1024K: 0.0203 against 0.0249 ms/iter (W = 1024)
-    {1280u * 1024, 256, 0},  // 1280K: 0.0285 against 0.0342 ms/iter (W = 1280)
-    {1296u * 1024, 2304, 0},  // 1296K: 0.0292 against 0.0410 ms/iter (W = 1024)
-    {1344u * 1024, 1024, 32},  // 1344K: 0.0322 against 0.0364 ms/iter (W = 1024)
-    {1440u * 1024, 2560, 0},  // 1440K: 0.0334 against 0.0424 ms/iter (W = 1024)
-    {1568u * 1024, 512, 0},  // 1568K: 0.0322 against 0.0373 ms/iter (W = 1024)
-    {1600u * 1024, 1024, 32},  // 1600K: 0.0373 against 0.0417 ms/iter (W = 1024)
-    {2160u * 1024, 512, 0},  // 2160K: 0.0474 against 0.0559 ms/iter (W = 1536)
-    {2880u * 1024, 2560, 0},  // 2880K: 0.0626 against 0.0794 ms/iter (W = 2048)
-    {3024u * 1024, 512, 0},  // 3024K: 0.0678 against 0.0768 ms/iter (W = 2304)
-    {3600u * 1024, 2304, 0},  // 3600K: 0.0879 against 0.0968 ms/iter (W = 1024)
-    {5120u * 1024, 1280, 0},  // 5120K: 0.0955 against 0.1032 ms/iter (W = 2048)
-    {7200u * 1024, 1280, 0},  // 7200K: 0.1653 against 0.1885 ms/iter (W = 2048)
-    {7776u * 1024, 1536, 0},  // 7776K: 0.1807 against 0.2043 ms/iter (W = 2048)
-    {9216u * 1024, 1536, 0},  // 9216K: 0.1826 against 0.1994 ms/iter (W = 2048)
-    {9408u * 1024, 3072, 0},  // 9408K: 0.2007 against 0.2243 ms/iter (W = 2048)
-    {10240u * 1024, 1280, 0},  // 10240K: 0.1980 against 0.2223 ms/iter (W = 2048)
-    {10800u * 1024, 2560, 0},  // 10800K: 0.2847 against 0.3449 ms/iter (W = 2304)
-    {12288u * 1024, 3072, 0},  // 12288K: 0.2316 against 0.2559 ms/iter (W = 2048)
-    {14336u * 1024, 1792, 0},  // 14336K: 0.2879 against 0.4295 ms/iter (W = 3584)
-    {16384u * 1024, 2048, 0},  // 16384K: 0.3229 against 0.4005 ms/iter (W = 4096)
-    {27216u * 1024, 4096, 0},  // 27216K: 0.8166 against 0.9911 ms/iter (W = 3584)
-    {28000u * 1024, 4096, 0},  // 28000K: 0.8687 against 1.0280 ms/iter (W = 3584)
-    {28672u * 1024, 4096, 0},  // 28672K: 0.7620 against 0.9017 ms/iter (W = 3584)
+    {112u * 1024, 512, 0},  // 112K: 0.0082 against 0.0089 ms/iter (W = 256)
+    {128u * 1024, 512, 0},  // 128K: 0.0075 against 0.0078 ms/iter (W = 256)
+    {160u * 1024, 512, 0},  // 160K: 0.0082 against 0.0085 ms/iter (W = 256)
+    {168u * 1024, 512, 0},  // 168K: 0.0089 against 0.0098 ms/iter (W = 256)
+    {224u * 1024, 512, 0},  // 224K: 0.0107 against 0.0114 ms/iter (W = 256)
+    {288u * 1024, 512, 32},  // 288K: four rows per CTA, as fast as two
+    {640u * 1024, 256, 0},  // 640K: 0.0161 against 0.0299 ms/iter (W = 1024)
+    {768u * 1024, 768, 0},  // 768K: 0.0181 against 0.0247 ms/iter (W = 512)
+    {784u * 1024, 256, 0},  // 784K: 0.0188 against 0.0237 ms/iter (W = 512)
+    {896u * 1024, 256, 0},  // 896K: 0.0201 against 0.0344 ms/iter (W = 1024)
+    {1024u * 1024, 512, 0},  // 1024K: 0.0187 against 0.0225 ms/iter (W = 1024)
+    {1152u * 1024, 1024, 32},  // 1152K: 0.0226 against 0.0287 ms/iter (W = 768)
+    {1280u * 1024, 256, 0},  // 1280K: 0.0266 against 0.0339 ms/iter (W = 1280)
+    {1296u * 1024, 2304, 0},  // 1296K: 0.0262 against 0.0389 ms/iter (W = 1024)
+    {1344u * 1024, 256, 0},  // 1344K: 0.0303 against 0.0344 ms/iter (W = 1024)
+    {1440u * 1024, 2560, 0},  // 1440K: 0.0290 against 0.0395 ms/iter (W = 1024)
+    {1568u * 1024, 1024, 32},  // 1568K: 0.0324 against 0.0356 ms/iter (W = 1024)
+    {1600u * 1024, 1024, 32},  // 1600K: 0.0372 against 0.0399 ms/iter (W = 1024)
+    {2160u * 1024, 512, 0},  // 2160K: 0.0467 against 0.0519 ms/iter (W = 1536)
+    {2304u * 1024, 512, 0},  // 2304K: 0.0380 against 0.0425 ms/iter (W = 768)
+    {2592u * 1024, 2304, 0},  // 2592K: 0.0509 against 0.0526 ms/iter (W = 768)
+    {2880u * 1024, 2560, 0},  // 2880K: 0.0567 against 0.0703 ms/iter (W = 2048)
+    {3584u * 1024, 512, 0},  // 3584K: 0.0590 against 0.0633 ms/iter (W = 1792)
+    {3600u * 1024, 2304, 0},  // 3600K: 0.0730 against 0.0891 ms/iter (W = 1024)
+    {4096u * 1024, 512, 0},  // 4096K: 0.0634 against 0.0672 ms/iter (W = 2048)
+    {7200u * 1024, 1280, 0},  // 7200K: 0.1620 against 0.1680 ms/iter (W = 2048)
+    {7776u * 1024, 2304, 0},  // 7776K: 0.1508 against 0.1815 ms/iter (W = 2048)
+    {8064u * 1024, 2304, 0},  // 8064K: 0.1350 against 0.1461 ms/iter (W = 1792)
+    {8640u * 1024, 2560, 0},  // 8640K: 0.1690 against 0.1855 ms/iter (W = 2048)
+    {9216u * 1024, 1536, 0},  // 9216K: 0.1418 against 0.1528 ms/iter (W = 2048)
+    {9408u * 1024, 3072, 0},  // 9408K: 0.1640 against 0.1992 ms/iter (W = 2048)
+    {10800u * 1024, 2560, 0},  // 10800K: 0.2413 against 0.2880 ms/iter (W = 2304)
+    {12544u * 1024, 3584, 0},  // 12544K: 0.2265 against 0.2385 ms/iter (W = 1792)
+    {14336u * 1024, 4096, 0},  // 14336K: 0.2403 against 0.2480 ms/iter (W = 3584)
+    {17496u * 1024, 2048, 0},  // 17496K: 0.3788 against 0.3976 ms/iter (W = 3072)
     {0, 0, 0},
 };
 
