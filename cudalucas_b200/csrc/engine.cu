@@ -1045,6 +1045,7 @@ struct ll_ctx {
   long long *carry = nullptr;
   uint32_t *flags = nullptr;
   DevState *st = nullptr;
+  DevState *host_st = nullptr;  // pinned copy for the read-back of a step
   double2 *twW = nullptr, *twH = nullptr, *thi = nullptr, *tlo = nullptr;
   double2 *stwW = nullptr, *stwH = nullptr;
   const PipeKernel *pipe_w = nullptr, *pipe_t = nullptr;  // persistent passes of plain iterations
@@ -1104,6 +1105,7 @@ static void free_ctx(ll_ctx *c) {
                   c->rowE, c->colF, c->rowW, c->rowWi, c->colW, c->colWi};
   for (void *p : ptrs)
     if (p) cudaFree(p);
+  if (c->host_st) cudaFreeHost(c->host_st);
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   if (c->graph) cudaGraphDestroy(c->graph);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -1303,7 +1305,8 @@ ll_status ll_create(int device, uint32_t q, uint32_t n, const ll_tuning *tuning,
         (e = cudaMalloc((void **)&ctx->xint, sizeof(int32_t) * (size_t)n)) != cudaSuccess ||
         (e = cudaMalloc((void **)&ctx->carry, carry_bytes)) != cudaSuccess ||
         (e = cudaMalloc((void **)&ctx->flags, flag_bytes)) != cudaSuccess ||
-        (e = cudaMalloc((void **)&ctx->st, sizeof(DevState))) != cudaSuccess) {
+        (e = cudaMalloc((void **)&ctx->st, sizeof(DevState))) != cudaSuccess ||
+        (e = cudaHostAlloc((void **)&ctx->host_st, sizeof(DevState), cudaHostAllocMapped)) != cudaSuccess) {
       rc = e == cudaErrorMemoryAllocation ? LL_ERR_NOMEM : cuda_fail(ctx, e, "cudaMalloc");
       break;
     }
@@ -1547,18 +1550,21 @@ static ll_status launch_init(ll_ctx *ctx) {
   return LL_OK;
 }
 
+// Enqueues the state of freshly loaded digits: the shift, no roundoff maximum,
+// no fault.  The counters are kept.
+static cudaError_t reset_state(ll_ctx *ctx, uint32_t offset) {
+  const uint32_t f[3] = {offset, 0u, 0u};
+  static_assert(offsetof(DevState, err_bits) == offsetof(DevState, offset) + 4 &&
+                    offsetof(DevState, fault) == offsetof(DevState, offset) + 8,
+                "offset, err_bits and fault are contiguous");
+  return cudaMemcpyAsync(&ctx->st->offset, f, sizeof f, cudaMemcpyHostToDevice, ctx->stream);
+}
+
 ll_status ll_load_digits(ll_ctx *ctx, const int32_t *digits, uint32_t offset) {
   if (!ctx || !digits || offset >= ctx->q) return LL_ERR_ARG;
   CK(cudaSetDevice(ctx->device));
   CK(cudaMemcpyAsync(ctx->xint, digits, sizeof(int32_t) * ctx->n, cudaMemcpyHostToDevice, ctx->stream));
-  DevState hs{};
-  // keep the ticket counter: read it back so that the whole struct can be rewritten
-  CK(cudaMemcpyAsync(&hs, ctx->st, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
-  hs.offset = offset;
-  hs.err_bits = 0;
-  hs.fault = 0;
-  CK(cudaMemcpyAsync(ctx->st, &hs, sizeof(DevState), cudaMemcpyHostToDevice, ctx->stream));
+  CK(reset_state(ctx, offset));
   ll_status rc = launch_init(ctx);
   if (rc != LL_OK) return rc;
   CK(cudaStreamSynchronize(ctx->stream));
@@ -1640,6 +1646,40 @@ static ll_status launch_cluster(ll_ctx *ctx, uint32_t iters, bool report) {
   return LL_OK;
 }
 
+// The read-back of a step: one small kernel writes the device state into pinned
+// host memory and restarts the roundoff maximum, instead of a pageable copy
+// back, its wait and a copy of the zero: 3136K checked after every iteration
+// 93.7 -> 85.0 us per iteration.
+static __global__ void report_state(DevState *st, DevState *host) {
+  *host = *st;
+  st->err_bits = 0;
+}
+
+static ll_status read_status(ll_ctx *ctx, float *max_err) {
+  DevState *dev = nullptr;
+  CK(cudaHostGetDevicePointer((void **)&dev, ctx->host_st, 0));
+  report_state<<<1, 1, 0, ctx->stream>>>(ctx->st, dev);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(ctx->stream));
+  const DevState hs = *ctx->host_st;
+  float e;
+  memcpy(&e, &hs.err_bits, sizeof(float));
+  if (max_err) *max_err = e;
+  if (hs.offset != ctx->offset) {
+    ctx->err = "device offset diverged from host mirror";
+    return LL_ERR_STATE;
+  }
+  if (hs.fault & 1u) {
+    ctx->err = "wide pass: carry wait timed out";
+    return LL_ERR_TIMEOUT;
+  }
+  if (hs.fault & 2u) {
+    ctx->err = "wide pass: a word beyond the exact FP64 range (roundoff far above 0.5, or digits out of range)";
+    if (max_err) *max_err = 1.0f;
+  }
+  return LL_OK;
+}
+
 ll_status ll_step(ll_ctx *ctx, uint32_t iters, uint32_t flags, float *max_err) {
   if (!ctx) return LL_ERR_ARG;
   if (!ctx->started) return LL_ERR_STATE;
@@ -1688,28 +1728,7 @@ ll_status ll_step(ll_ctx *ctx, uint32_t iters, uint32_t flags, float *max_err) {
     if (rc != LL_OK) return rc;
   }
   if (iters) ctx->digits_current = report;
-  if ((flags & (LL_REPORT | LL_ERRCHK)) && !(flags & LL_ASYNC)) {
-    DevState hs{};
-    CK(cudaMemcpyAsync(&hs, ctx->st, sizeof(DevState), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    const uint32_t zero[2] = {0, 0};
-    CK(cudaMemcpyAsync(&ctx->st->err_bits, zero, sizeof(uint32_t), cudaMemcpyHostToDevice, ctx->stream));
-    float e;
-    memcpy(&e, &hs.err_bits, sizeof(float));
-    if (max_err) *max_err = e;
-    if (hs.offset != ctx->offset) {
-      ctx->err = "device offset diverged from host mirror";
-      return LL_ERR_STATE;
-    }
-    if (hs.fault & 1u) {
-      ctx->err = "wide pass: carry wait timed out";
-      return LL_ERR_TIMEOUT;
-    }
-    if (hs.fault & 2u) {
-      ctx->err = "wide pass: a word beyond the exact FP64 range (roundoff far above 0.5, or digits out of range)";
-      if (max_err) *max_err = 1.0f;
-    }
-  }
+  if ((flags & (LL_REPORT | LL_ERRCHK)) && !(flags & LL_ASYNC)) return read_status(ctx, max_err);
   return LL_OK;
 }
 
@@ -1732,12 +1751,7 @@ ll_status ll_device_restore(ll_ctx *ctx, uint32_t *offset) {
   if (!ctx->ck_valid) return LL_ERR_STATE;
   CK(cudaSetDevice(ctx->device));
   CK(cudaMemcpyAsync(ctx->xint, ctx->ck_digits, sizeof(int32_t) * ctx->n, cudaMemcpyDeviceToDevice, ctx->stream));
-  // offset, roundoff maximum and fault bits; the ticket counter is kept
-  const uint32_t f[3] = {ctx->ck_offset, 0u, 0u};
-  static_assert(offsetof(DevState, err_bits) == offsetof(DevState, offset) + 4 &&
-                    offsetof(DevState, fault) == offsetof(DevState, offset) + 8,
-                "offset, err_bits and fault are contiguous");
-  CK(cudaMemcpyAsync(&ctx->st->offset, f, sizeof f, cudaMemcpyHostToDevice, ctx->stream));
+  CK(reset_state(ctx, ctx->ck_offset));
   const ll_status rc = launch_init(ctx);
   if (rc != LL_OK) return rc;
   ctx->offset = ctx->ck_offset;
@@ -2376,16 +2390,22 @@ ll_status ll_batch_step(ll_batch *b, uint32_t iters, uint32_t flags, float *max_
     cudaEventRecord(b->events[0], b->stream);
     for (ll_ctx *c : b->members) cudaStreamWaitEvent(c->stream, b->events[0], 0);
   }
-  for (size_t i = 0; i < b->members.size(); ++i) {
-    ll_ctx *c = b->members[i];
-    float e = 0.f;
-    const uint32_t rest = iters - done;
+  // the remaining iterations of all members are enqueued before any is waited
+  // for, so that they overlap
+  const uint32_t rest = iters - done;
+  for (ll_ctx *c : b->members) {
     if (rest || flags) {
-      ll_status s = ll_step(c, rest, flags, &e);
+      const ll_status s = ll_step(c, rest, flags | LL_ASYNC, nullptr);
       if (s != LL_OK) return s;
     } else if (iters) {
       c->digits_current = false;
     }
+  }
+  const bool wait = (flags & (LL_REPORT | LL_ERRCHK)) && !(flags & LL_ASYNC);
+  for (size_t i = 0; i < b->members.size(); ++i) {
+    float e = 0.f;
+    const ll_status s = wait ? read_status(b->members[i], &e) : LL_OK;
+    if (s != LL_OK) return s;
     if (max_err) max_err[i] = e;
   }
   return LL_OK;
