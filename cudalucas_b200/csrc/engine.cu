@@ -464,6 +464,10 @@ using L4096 = RList<16, 16, 16>;
 // column lengths of the tall_any kernels
 using C24 = RList<4, 6>;
 using C28 = RList<4, 7>;
+using C64 = RList<8, 8>;
+using C72 = RList<9, 8>;
+using C84 = RList<12, 7>;
+using C96 = RList<12, 8>;
 using C100 = RList<10, 10>;
 using C112 = RList<16, 7>;
 using C120 = RList<12, 10>;
@@ -567,6 +571,8 @@ static const StaticTall kTall[] = {
     LLB_TALL(L256),  LLB_TALL(L512),  LLB_TALL(L768),  LLB_TALL(L1024), LLB_TALL(L1280), LLB_TALL(L1536), LLB_TALL(L1792),
     LLB_TALL(L2048), LLB_TALL(L2304), LLB_TALL(L2560), LLB_TALL(L3072), LLB_TALL(L3584), LLB_TALL(L4096),
     LLB_TALL_ANY(C24, 6, 1),        LLB_TALL_ANY(C28, 7, 1),
+    LLB_TALL_ANY(C64, 8, 1),        LLB_TALL_ANY(C72, 9, 1),
+    LLB_TALL_ANY(C84, 12, 1),       LLB_TALL_ANY(C96, 12, 1),
     LLB_TALL_ANY(C100, 10, 1),      LLB_TALL_ANY(C112, 8, 1),
     LLB_TALL_ANY(C120, 12, 1),      LLB_TALL_ANY(C128, 16, 2),
     LLB_TALL_ANY(C140, 14, 1),
@@ -676,23 +682,19 @@ struct ClusterKernel {
   int tw;              // stage twiddle entries of both lists
   int threads;         // per CTA
   int smem;            // dynamic shared-memory entries
+  uint32_t most;       // used for steps of fewer iterations only (0: for every step)
 };
 #define LLB_CRAD(LIST)                                                                                \
   LIST::N, {LIST::a[0], LIST::N > 1 ? LIST::a[1 % LIST::N] : 0, LIST::N > 2 ? LIST::a[2 % LIST::N] : 0, \
             LIST::N > 3 ? LIST::a[3 % LIST::N] : 0}
-#define LLB_CLUSTER(PR, TWR, LT, TC, C, RPC)                                                                     \
+#define LLB_CLUSTER_FEW(PR, TWR, LT, TC, C, RPC, MOST)                                                                     \
   {PR::L, LT::L, C, cluster_iters<PR, TWR, LT, TC, C, RPC>, LLB_RAD(PR), LLB_CRAD(LT), tw_size<PR>() + tw_size<LT>(), \
-   ClusterCfg<PR, TWR, LT, TC, C, RPC>::T, ClusterCfg<PR, TWR, LT, TC, C, RPC>::total}
+   ClusterCfg<PR, TWR, LT, TC, C, RPC>::T, ClusterCfg<PR, TWR, LT, TC, C, RPC>::total, MOST}
+#define LLB_CLUSTER(PR, TWR, LT, TC, C, RPC) LLB_CLUSTER_FEW(PR, TWR, LT, TC, C, RPC, 0)
 // row lists of 256: 64 threads per row (one radix-4 butterfly each per
 // stage) or 32 threads per row
 using R256A = RList<4, 4, 4, 4>;
 using R256B = RList<8, 4, 8>;
-// rows of 768 and 1024: 192 and 256 threads per row (both directions run the
-// list in the same order, so it need not be palindromic)
-using R768 = RList<4, 6, 8, 4>;
-using R1024 = RList<4, 8, 8, 4>;
-using R768B = RList<8, 12, 8>;    // 96 threads per row
-using R1024B = RList<8, 16, 8>;   // 128 threads per row
 // column lists of small radices: many threads per column, short chains
 using K16 = RList<4, 4>;
 using K20 = RList<4, 5>;
@@ -702,24 +704,26 @@ using K32 = RList<4, 8>;
 using K36 = RList<6, 6>;
 using K40 = RList<5, 8>;
 using K64 = RList<4, 4, 4>;
+using K72 = RList<8, 9>;
+using K84 = RList<7, 12>;
+using K96 = RList<8, 12>;
 using K112 = RList<4, 4, 7>;
-// Only lengths where one cluster (16 SMs) beats two launches over the whole
-// GPU (us per iteration, cluster against two launches): 8K 3.6 / 13.4, 10K
-// 5.1 / 15.6, 12K 4.8 / 9.9, 14K 5.7 / 10.0, 16K 4.8 / 17.2, 18K 6.1 / 17.7,
-// 20K 6.5 / 16.3, 32K 7.8 / 16.5, 56K 13.1 / 14.8, and with rows of 768 and
-// 1024: 36K 11.6 / 16.1, 42K 12.9 / 16.3, 48K 14.5 / 21.7.  At 50K (15.7 /
-// 11.7) and 96K (21.7 / 12.1) the arithmetic of 16 SMs is the bound and the
-// two-launch path stays.
+// Up to 20K one cluster (16 SMs) runs every step (8K 3.5, 12K 4.4, 16K 4.8, 20K
+// 6.3 us per iteration).  From 32K on the arithmetic of 16 SMs is the bound
+// and two launches over the whole GPU win (cluster against two launches: 32K
+// 7.4 / 5.8, 36K 10.8 / 6.2, 42K 12.1 / 6.5, 48K 13.6 / 6.4, 56K 12.4 / 6.9);
+// there the cluster runs the steps of fewer than kFewIters iterations, as one
+// launch.
+constexpr uint32_t kFewIters = 8;
 static const ClusterKernel kCluster[] = {
     LLB_CLUSTER(R256A, 64, K16, 4, 16, 1),    LLB_CLUSTER(R256B, 32, K20, 5, 16, 2),
     LLB_CLUSTER(R256A, 64, K24, 6, 16, 2),    LLB_CLUSTER(R256B, 32, K24, 6, 16, 2),
     LLB_CLUSTER(R256A, 64, K24, 6, 8, 4),     LLB_CLUSTER(R256B, 32, K28, 7, 16, 2),
     LLB_CLUSTER(R256A, 64, K28, 7, 8, 4),     LLB_CLUSTER(R256A, 64, K32, 8, 16, 2),
     LLB_CLUSTER(R256B, 32, K36, 6, 16, 3),    LLB_CLUSTER(R256A, 64, K40, 8, 16, 4),
-    LLB_CLUSTER(R256A, 64, K64, 16, 16, 4),   LLB_CLUSTER(R256B, 32, K112, 28, 16, 8),
-    LLB_CLUSTER(R768, 192, K24, 6, 16, 2),    LLB_CLUSTER(R768B, 96, K24, 6, 16, 2),
-    LLB_CLUSTER(R768B, 96, K28, 8, 16, 2),    LLB_CLUSTER(R768, 192, K28, 8, 16, 2),
-    LLB_CLUSTER(R1024B, 128, K24, 6, 16, 2),  LLB_CLUSTER(R1024, 256, K24, 6, 16, 2),
+    LLB_CLUSTER_FEW(R256A, 64, K64, 16, 16, 4, kFewIters), LLB_CLUSTER_FEW(R256B, 32, K72, 10, 16, 6, kFewIters),
+    LLB_CLUSTER_FEW(R256B, 32, K84, 12, 16, 6, kFewIters), LLB_CLUSTER_FEW(R256B, 32, K96, 12, 16, 6, kFewIters),
+    LLB_CLUSTER_FEW(R256B, 32, K112, 28, 16, 8, kFewIters),
 };
 
 static const StaticTall *find_tall(int L) {
@@ -1692,7 +1696,7 @@ ll_status ll_step(ll_ctx *ctx, uint32_t iters, uint32_t flags, float *max_err) {
   const bool report = (flags & LL_REPORT) != 0;
   uint32_t done = 0;
   const uint32_t K = (uint32_t)ctx->graph_iters;
-  if (ctx->cluster && iters) {
+  if (ctx->cluster && iters && (!ctx->cluster->most || iters < ctx->cluster->most)) {
     const ll_status rc = launch_cluster(ctx, iters, report);
     if (rc != LL_OK) return rc;
     done = iters;
@@ -2150,8 +2154,8 @@ extern "C" ll_status ll_step_static(int device, uint32_t q, uint32_t n, uint32_t
 // shape).  One step of K iterations for the whole batch is a single CUDA
 // graph: each member's chain of K x (tall, wide) launches is its own branch,
 // the branches fork from and join back to the batch stream, and the GPU runs
-// the independent branches concurrently.  A member runs exactly the kernels it
-// would run alone, so its residues are the solo residues.
+// the independent branches concurrently.  A member runs the kernels that
+// a context of its tuning would run alone, so its residues are the solo residues.
 // Members of one FFT length whose passes both have specialised kernels run
 // as a length class: one launch per pass for all of them (blockIdx.x =
 // member * units + unit), the members' kernel arguments in a device array.
@@ -2253,7 +2257,6 @@ static ll_status build_classes(ll_batch *b) {
   return LL_OK;
 }
 
-constexpr int kBatchCarveout = 100;
 static void launch_class(const void *kern, const void *arr, int units, int count, int threads, size_t smem,
                          cudaStream_t st, bool chained) {
   cudaLaunchConfig_t cfg = {};
@@ -2262,7 +2265,7 @@ static void launch_class(const void *kern, const void *arr, int units, int count
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
-  pass_attributes(cfg, attr, chained, kBatchCarveout);
+  pass_attributes(cfg, attr, chained, -1);
   void *argv[] = {(void *)&arr, (void *)&units};
   cudaLaunchKernelExC(&cfg, kern, argv);
 }
@@ -2278,6 +2281,11 @@ ll_status ll_batch_create(int device, int32_t count, const uint32_t *q, const ui
   b->graph_iters = graph_iters > 0 ? graph_iters : 10;
   ll_tuning t{};
   t.graph_iters = -1;  // members never capture their own graphs
+  // A batch is bound by the work of all members together, not by the latency
+  // of a pass: it takes the 16-element rows nearest sqrt(N) rather than what is
+  // fastest alone (32 members of 50K to 1024K, 390 iterations: 91.6 ms with the
+  // solo choice, 81.4 with this).
+  t.kernels = LL_KERNELS_NO_CLUSTER;
   for (int32_t i = 0; i < count; ++i) {
     ll_ctx *c = nullptr;
     ll_status s = ll_create(device, q[i], n[i], &t, &c);

@@ -67,8 +67,9 @@ typedef struct {
  * (measured slower at 12K and 14K, equal at 56K, so not the default);
  * LL_KERNELS_NO_PREFETCH turns off the L2 prefetch that lengths larger than
  * L2 use.  Short lengths with a cluster-resident kernel (8K, 10K, 12K, 14K,
- * 16K, 18K, 20K, 32K, 36K, 42K, 48K, 56K) run each ll_step as one launch of
- * one thread-block cluster whose shared memory holds the whole state;
+ * 16K, 18K, 20K; 32K, 36K, 42K, 48K, 56K for steps of fewer than 8 iterations)
+ * run an ll_step as one launch of one thread-block cluster whose shared memory
+ * holds the whole state;
  * LL_KERNELS_NO_CLUSTER turns that off (two launches per iteration),
  * LL_KERNELS_CLUSTER8 keeps to the portable cluster size of 8 CTAs. */
 #define LL_KERNELS_GENERIC 1
@@ -77,7 +78,9 @@ typedef struct {
 #define LL_KERNELS_NO_CLUSTER 8   /* no cluster-resident iterations */
 #define LL_KERNELS_CLUSTER8 16    /* clusters of at most 8 CTAs */
 #define LL_KERNELS_ALT_WIDE 32    /* the alternative row kernel where a length has one
-                                     (rows in shared memory, 8 elements per thread) */
+                                     (rows in shared memory, 8 elements per thread);
+                                     with any of these flags short lengths run the
+                                     rows of 16 elements per thread */
 
 /* Creates a context for exponent q at FFT length n (FP64 words) on `device`.
  * With tuning NULL (or all zero) the engine chooses the launch: for some
@@ -147,9 +150,9 @@ void ll_shape(const ll_ctx *ctx, int32_t *width, int32_t *height,
 const char *ll_last_error(const ll_ctx *ctx); /* text of the last failure   */
 /* Which passes run compile-time specialised kernels: bit 0 the wide (row)
  * pass, bit 1 the tall (column) pass (the others use the generic kernels);
- * bit 2: plain iterations run as fused cooperative launches; bit 3: every
- * step runs as cluster-resident launches (the state in the shared memory of
- * one thread-block cluster). */
+ * bit 2: plain iterations run as fused cooperative launches; bit 3: steps
+ * run as cluster-resident launches (the state in the shared memory of one
+ * thread-block cluster; from 32K on the steps of fewer than 8 iterations). */
 int32_t ll_kernel_kinds(const ll_ctx *ctx);
 /* Host-only self-check of the compiled kernel tables: the number of
  * specialised kernels whose stage-twiddle table (built on the host from the
@@ -174,7 +177,8 @@ ll_status ll_debug_launch(ll_ctx *ctx, int32_t which);
  * ll_read_digits, ...); one step of `graph_iters` iterations of all members is
  * replayed from a single CUDA graph in which every member is a parallel
  * branch, so members of different lengths overlap on the GPU.  A member runs
- * exactly the kernels of a solo run: its residues equal the solo residues. */
+ * the kernels of a solo run with LL_KERNELS_NO_CLUSTER: its residues equal the
+ * solo residues. */
 typedef struct ll_batch ll_batch;
 ll_status ll_batch_create(int device, int32_t count, const uint32_t *q, const uint32_t *n, int32_t graph_iters,
                           ll_batch **out);
