@@ -945,16 +945,30 @@ std::vector<double2> stage_twiddles(const int *rad, int nrad) {
 
 }  // namespace
 
+// tan(2*pi*num/den), from the nearer end of the quarter turn.
+static double tangent(unsigned long long num, unsigned long long den) {
+  const long double PI = 3.14159265358979323846264338327950288L;
+  const unsigned long long n4 = num % den * 4, quarter = n4 / den, rem = n4 - quarter * den;
+  const bool upper = 2 * rem > den;
+  long double t = tanl((long double)(upper ? den - rem : rem) / (long double)den * (PI / 2));
+  if (upper) t = 1 / t;
+  return (double)(quarter & 1 ? -1 / t : t);
+}
+
 // Twiddle table of the persistent passes for length L = 256*M (see
-// kernels_pipe.cuh): entry e < 8 of thread c at [e*TR + c], then the stage-1
-// twiddles w_TR^(j0*v) at rows of odd stride.
+// kernels_pipe.cuh): entry e < 8 of thread c, as cosine and tangent, at
+// [e*TR + c], then the stage-1 twiddles w_TR^(j0*v) at rows of odd stride.
 static std::vector<double2> pipe_twiddles(int L) {
   const int M = L / 256, TR = L / 16, SS = M | 1;
   std::vector<double2> out((size_t)8 * TR + (M > 1 ? 16 * SS : 0), make_double2(0.0, 0.0));
   static const int power[8] = {8, 4, 2, 2, 1, 1, 1, 1}, root[8] = {0, 0, 0, 2, 0, 1, 2, 3};
   for (int c = 0; c < TR; ++c)
-    for (int e = 0; e < 8; ++e)
-      out[(size_t)e * TR + c] = unit_root((unsigned long long)power[e] * c + (unsigned long long)root[e] * (L / 16), L);
+    for (int e = 0; e < 8; ++e) {
+      const int num = power[e] * c + root[e] * (L / 16);  // less than half a turn
+      // the quarter turn: a cosine far below rounding keeps the tangent finite
+      out[(size_t)e * TR + c] = 4 * num == L ? make_double2(0x1p-60, 0x1p60)
+                                             : make_double2(unit_root(num, L).x, tangent(num, L));
+    }
   if (M > 1)
     for (int j = 0; j < 16; ++j)
       for (int v = 0; v < M; ++v) out[(size_t)8 * TR + j * SS + v] = unit_root((unsigned long long)j * v, TR);

@@ -51,20 +51,22 @@ struct Pipe {
   static_assert(NS >= NG && NS >= 1, "a slot per group");
 };
 
-// Twiddle table of a length: entry e < 8 of thread c at [e*TR + c], the powers
-// of z = w_L^c that dft16_tw takes: z^8, z^4, z^2, z^2*w8, z, z*w16, z*w8,
-// z*w16^3; then the stage-1 twiddles w_TR^(j0*v) at [8*TR + j0*SS + v].
+// Twiddle table of a length: entry e < 8 of thread c at [e*TR + c], cosine and
+// tangent of the powers of z = w_L^c that dft16_tw takes: z^8, z^4, z^2,
+// z^2*w8, z, z*w16, z*w8, z*w16^3; then the stage-1 twiddles w_TR^(j0*v) at [8*TR + j0*SS + v].
 
-// a + e*b and a - e*b (the latter as 2a - (a + e*b)): six fused operations.
+// a + e*b and a - e*b in six fused operations; w.x is the cosine, w.y the
+// tangent of the twiddle: e*b = c*(b + i*t*b), so each result has two
+// roundings.  (With a - e*b as 2a - (a + e*b) it has three: a transform of 3072
+// then has an rms error of 2.08 units, this 1.99, products and dft16 1.97.)
 // e = w, or i*w with ROT; conjugated for SIGN < 0.
 template <int SIGN, bool ROT>
 __device__ __forceinline__ void bfly(double2 &a, double2 &b, double2 w) {
-  const double ex = ROT ? -w.y : w.x;
-  const double ey = SIGN > 0 ? (ROT ? w.x : w.y) : (ROT ? -w.x : -w.y);
-  const double px = fma(ex, b.x, fma(-ey, b.y, a.x));
-  const double py = fma(ex, b.y, fma(ey, b.x, a.y));
-  b = make_double2(fma(2.0, a.x, -px), fma(2.0, a.y, -py));
-  a = make_double2(px, py);
+  const double c = w.x, t = SIGN > 0 ? w.y : -w.y;
+  const double ux = fma(-t, b.y, b.x), uy = fma(t, b.x, b.y);  // w*b = c*u
+  const double rx = ROT ? (SIGN > 0 ? -uy : uy) : ux, ry = ROT ? (SIGN > 0 ? ux : -ux) : uy;
+  b = make_double2(fma(-c, rx, a.x), fma(-c, ry, a.y));
+  a = make_double2(fma(c, rx, a.x), fma(c, ry, a.y));
 }
 
 // 16-point DFT of v[r]*z^r in 192 fused operations (60 of complex products
@@ -320,9 +322,8 @@ __device__ __forceinline__ void pipe_second(unsigned char *sm, const C cells, co
 
 // ------------------------------------------------------------- tall pass --
 // Constants of a column pair: for both columns the 16 factors g^r = w_N^(k*TR*r)
-// of the stores and g^2*w8, g*w16, g*w8, g*w16^3 (with g^8, g^4, g^2, g the
-// table of dft16_tw), and w_N^kA of the pairing.
-constexpr int kPairConst = 41;
+// of the column twiddles, and w_N^kA of the pairing.
+constexpr int kPairConst = 33;
 
 template <int M>
 constexpr int tall_pipe_smem() {
@@ -356,11 +357,8 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1) tall_pipe(const __grid_constan
   // Constants of pair u, entry i: product of two table entries, fetched into
   // shared memory (raw) while the unit before is worked on.
   auto constant_exp = [&](int u, int i) {
-    if (i == 40) return u;
-    const int kk = i < 20 ? u : u == 0 ? W / 2 : W - u, j = i < 20 ? i : i - 20, n16 = a.N / 16;
-    if (j < 16) return kk * TR * j;
-    const int e = j == 16 ? kk * TR * 2 + 2 * n16 : kk * TR + (j - 16) * n16;
-    return e >= a.N ? e - a.N : e;
+    if (i == 32) return u;
+    return (i < 16 ? u : u == 0 ? W / 2 : W - u) * TR * (i & 15);
   };
   auto fill = [&](int u, int pos) {  // one thread
     const int slot = pos % NS;
@@ -433,23 +431,22 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1) tall_pipe(const __grid_constan
     double2 v[16];
 #pragma unroll
     for (int r = 0; r < 16; ++r) v[r] = cell(smb, cells.base + (uint32_t)(t + r * TR) * 16);
-    const double2 *gc = cst + 20 * col;
-    dft16_tw<+1>(v, [&](int e) {
-      return gc[e == 0 ? 8 : e == 1 ? 4 : e == 2 ? 2 : e == 3 ? 16 : e == 4 ? 1 : 12 + e];
-    });
+    const double2 *gc = cst + 16 * col;
+    // each element times its own twiddle: folded into the transform's layers
+    // the factors are products of four rounded ones
     const double2 base = cmul(bh, bl);
 #pragma unroll
-    for (int r = 0; r < 16; ++r) v[r] = cmul(v[r], base);
-    auto bitrev = [](int r) { return slot16(r); };
+    for (int r = 0; r < 16; ++r) v[r] = cmul(v[r], cmul(base, gc[r]));
+    dft16<+1>(v);
     auto ord16 = [](int r) { return out_slot<16>(r); };
-    pipe_first<M, +1>(smb, cells, tw, t, cells1, it0, v, bitrev, sync);
+    pipe_first<M, +1>(smb, cells, tw, t, cells1, it0, v, ord16, sync);
     if (NS > NG) refill();
     if (!special) {
       // bin c + r*TR of column kA pairs with bin (TR-1-c) + (15-r)*TR of
       // column kB, held by the neighbouring lane: each lane takes the lower
       // half of its own bins.  Swapping the two bins and conjugating w swaps
       // the results, so both lanes make the same call.
-      const double2 wb = cmul(cst[40], wh);
+      const double2 wb = cmul(cst[32], wh);
       const double sg = col ? -1.0 : 1.0;
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
