@@ -1005,7 +1005,7 @@ static const PreferredShape kPreferred[] = {
     {1296u * 1024, 2304, 0},  // 1296K: 0.0262 against 0.0389 ms/iter (W = 1024)
     {1344u * 1024, 256, 0},  // 1344K: 0.0303 against 0.0344 ms/iter (W = 1024)
     {1440u * 1024, 2560, 0},  // 1440K: 0.0290 against 0.0395 ms/iter (W = 1024)
-    {1568u * 1024, 1024, 32},  // 1568K: 0.0324 against 0.0356 ms/iter (W = 1024)
+    {1568u * 1024, 512, 0},  // 1568K: 0.0323 against 0.0356 ms/iter (W = 1024)
     {1600u * 1024, 1024, 32},  // 1600K: 0.0372 against 0.0399 ms/iter (W = 1024)
     {2160u * 1024, 512, 0},  // 2160K: 0.0467 against 0.0519 ms/iter (W = 1536)
     {2304u * 1024, 512, 0},  // 2304K: 0.0380 against 0.0425 ms/iter (W = 768)
