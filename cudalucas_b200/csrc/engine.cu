@@ -90,6 +90,7 @@ struct TallArgs {
   int W, H, N, ts, tmask;
   uint32_t q;
   int pf;  // > 0: prefetch into L2 the column pair pf units ahead (state larger than L2)
+  long long wait;  // limit of the waits inside a pass, in cycles
 };
 
 struct WideArgs {
@@ -112,6 +113,7 @@ struct WideArgs {
   int W, H, G, ngroups;
   int chains, chain_len;  // persistent row pass: runs of units that advance side by side
   int pf;  // > 0: prefetch into L2 the row group pf tickets ahead (state larger than L2)
+  long long wait;  // limit of the waits inside a pass, in cycles (specialised kernels)
   uint32_t q, n, b, qn;
   double inv_q, inv_n, inv_H;  // reciprocals for udiv_est
   // specialised kernels: column m1 = t + r*TR has exponent colF[t] - D_r
@@ -1459,7 +1461,7 @@ ll_status ll_create(int device, uint32_t q, uint32_t n, const ll_tuning *tuning,
     }
     TallArgs &ta = ctx->ta;
     ta.A = ctx->A; ta.ptw = ctx->ptwH; ta.stw = ctx->stwH; ta.twH = ctx->twH; ta.thi = ctx->thi; ta.tlo = ctx->tlo; ta.st = ctx->st;
-    ta.ph = ctx->ph; ta.W = s.W; ta.H = s.H; ta.N = ctx->N; ta.ts = ctx->ts; ta.tmask = (1 << ctx->ts) - 1; ta.q = q;
+    ta.ph = ctx->ph; ta.W = s.W; ta.H = s.H; ta.N = ctx->N; ta.ts = ctx->ts; ta.tmask = (1 << ctx->ts) - 1; ta.q = q; ta.wait = kWaitCycles;
     WideArgs &wa = ctx->wa;
     if (ctx->pipe_w) {
       // a multiple of the slots, about 32, of four units or more each
@@ -1472,7 +1474,7 @@ ll_status ll_create(int device, uint32_t q, uint32_t n, const ll_tuning *tuning,
     wa.rowE = ctx->rowE; wa.rowW = ctx->rowW; wa.rowWi = ctx->rowWi;
     wa.colF = ctx->colF; wa.colW = ctx->colW; wa.colWi = ctx->colWi;
     wa.st = ctx->st; wa.pw = ctx->pw; wa.W = s.W; wa.H = s.H; wa.G = s.G; wa.ngroups = ngroups;
-    wa.q = q; wa.n = n; wa.b = ctx->b; wa.qn = ctx->qn;
+    wa.q = q; wa.n = n; wa.b = ctx->b; wa.qn = ctx->qn; wa.wait = kWaitCycles;
     // A state larger than half of L2 is read from HBM by every pass: each CTA
     // prefetches into L2 the unit about one wave ahead (the CTAs resident at
     // once), so that unit's loads hit L2.
@@ -1895,6 +1897,19 @@ void ll_debug_inject_failure(ll_ctx *ctx, int32_t count) {
   if (ctx) ctx->inject = count;
 }
 
+ll_status ll_debug_wait_limit(ll_ctx *ctx, int64_t cycles) {
+  if (!ctx) return LL_ERR_ARG;
+  CK(cudaSetDevice(ctx->device));
+  CK(cudaStreamSynchronize(ctx->stream));
+  ctx->ta.wait = ctx->wa.wait = cycles ? cycles : kWaitCycles;
+  // the step graph holds the kernels' arguments: it is captured again
+  if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
+  if (ctx->graph) cudaGraphDestroy(ctx->graph);
+  ctx->graph_exec = nullptr;
+  ctx->graph = nullptr;
+  return LL_OK;
+}
+
 ll_status ll_debug_launch(ll_ctx *ctx, int32_t which) {
   if (!ctx || !ctx->started) return LL_ERR_STATE;
   CK(cudaSetDevice(ctx->device));
@@ -2108,14 +2123,14 @@ extern "C" ll_status ll_step_static(int device, uint32_t q, uint32_t n, uint32_t
   TallArgs ta{};
   ta.A = A; ta.stw = (const double2 *)dev(h_stwH); ta.twH = (const double2 *)dev(h_twH);
   ta.thi = (const double2 *)dev(h_hi); ta.tlo = (const double2 *)dev(h_lo); ta.st = dst;
-  ta.ph = ph; ta.W = W; ta.H = H; ta.N = N; ta.ts = ts; ta.tmask = (1 << ts) - 1; ta.q = q;
+  ta.ph = ph; ta.W = W; ta.H = H; ta.N = N; ta.ts = ts; ta.tmask = (1 << ts) - 1; ta.q = q; ta.wait = kWaitCycles;
   WideArgs wa{};
   wa.A = A; wa.stw = (const double2 *)dev(h_stwW); wa.carry = carry; wa.flags = flags;
   wa.twW = (const double2 *)dev(h_twW);
   wa.rowE = (const int32_t *)dev(h_rE); wa.rowW = (const double *)dev(h_rW); wa.rowWi = (const double *)dev(h_rWi);
   wa.colF = (const int32_t *)dev(h_cF); wa.colW = (const double *)dev(h_cW); wa.colWi = (const double *)dev(h_cWi);
   wa.st = dst; wa.pw = pw; wa.W = W; wa.H = H; wa.G = s.G; wa.ngroups = ngroups;
-  wa.q = q; wa.n = n; wa.b = b; wa.qn = qn;
+  wa.q = q; wa.n = n; wa.b = b; wa.qn = qn; wa.wait = kWaitCycles;
   fill_wide_constants(wa, s);
 
   // ---- state that must start at zero: flags, ticket, error, fault

@@ -135,8 +135,10 @@ struct GroupSync {
 // had not come by then the group waits for that thread.  Since the group goes
 // by one thread's word, a wait that runs out (it is bounded, sets the timeout
 // fault bit and makes every later wait of the CTA give up at once) ends the
-// group's work without leaving any of its threads behind at a barrier.
-constexpr int kNotYet = -9;
+// group's work without leaving any of its threads behind at a barrier.  A
+// group that gives up draws no more units and touches no slot; the copies that
+// its CTA has asked for by then are waited for before the CTA leaves (drain).
+constexpr int kNotYet = -9, kGaveUp = -10;
 __device__ __forceinline__ uint32_t smem32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void slot_init(uint64_t *bar) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem32(bar)) : "memory");
@@ -160,14 +162,14 @@ __device__ __forceinline__ bool slot_full(uint64_t *bar, uint32_t parity) {
 // group is behind); the parity alone would then take the phase before that for
 // its own.
 __device__ __forceinline__ bool slot_wait(uint64_t *bar, uint32_t parity, volatile int *pos_of, int pos, DevState *st,
-                                          volatile int *dead) {
+                                          volatile int *dead, long long limit) {
   long long t0 = 0;
   for (int k = 0;; ++k) {
     if (*pos_of == pos && slot_full(bar, parity)) return true;
     if (*dead) return false;
     const long long now = clock64();
     if (k == 0) t0 = now;
-    else if (now - t0 > kWaitCycles) {
+    if (now - t0 > limit) {
       *dead = 1;
       atomicOr(&st->fault, 1u);
       return false;
@@ -175,7 +177,7 @@ __device__ __forceinline__ bool slot_wait(uint64_t *bar, uint32_t parity, volati
   }
 }
 // Waits (bounded) until the flag is up and takes it down.
-__device__ __forceinline__ void await_extra(uint32_t *flag, DevState *st, volatile int *dead) {
+__device__ __forceinline__ void await_extra(uint32_t *flag, DevState *st, volatile int *dead, long long limit) {
   long long t0 = 0;
   for (int k = 0;; ++k) {
     uint32_t v;
@@ -183,13 +185,23 @@ __device__ __forceinline__ void await_extra(uint32_t *flag, DevState *st, volati
     if (v || *dead) break;
     const long long now = clock64();
     if (k == 0) t0 = now;
-    else if (now - t0 > kWaitCycles) {
+    if (now - t0 > limit || ((k & 1023) == 1023 && (*(volatile uint32_t *)&st->fault & 1u))) {
       *dead = 1;
       atomicOr(&st->fault, 1u);
       break;
     }
   }
   *flag = 0;
+}
+// After a wait has run out: the copy that the slot was last filled by has
+// landed before the CTA leaves its shared memory to another one (one thread
+// per slot, all fills issued; bounded by itself, whatever the limit of the
+// other waits).  pos < 0: never filled.
+__device__ __forceinline__ void drain(uint64_t *bar, int pos, int slots) {
+  if (pos < 0) return;
+  const long long t0 = clock64();
+  while (!slot_full(bar, (uint32_t)(pos / slots) & 1u) && clock64() - t0 < kWaitCycles) {
+  }
 }
 __device__ __forceinline__ void copy_bulk(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
   asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem32(dst)),
@@ -351,7 +363,10 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1) tall_pipe(const __grid_constan
   for (int i = threadIdx.x; i < P::TWN; i += P::NT) cp_async16(&tw[i], &a.ptw[i]);
   if (threadIdx.x == 0) {
     s_dead = 0;
-    for (int s = 0; s < NS; ++s) slot_init(&full[s]);
+    for (int s = 0; s < NS; ++s) {
+      s_pos[s] = -1;
+      slot_init(&full[s]);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // Constants of pair u, entry i: product of two table entries, fetched into
@@ -422,7 +437,7 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1) tall_pipe(const __grid_constan
     int go = pos == g ? kNotYet : s_go[g];
     if (go == kNotYet) {
       sync();
-      if (idx == TU - 1) s_go[g] = slot_wait(&full[slot], parity, &s_pos[slot], pos, a.st, &s_dead);
+      if (idx == TU - 1) s_go[g] = slot_wait(&full[slot], parity, &s_pos[slot], pos, a.st, &s_dead, a.wait);
       sync();
       go = s_go[g];
     }
@@ -525,8 +540,11 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1) tall_pipe(const __grid_constan
     }
   }
   // a refill that is still due belongs to another group's next unit
-  refill();
+  if (!*(volatile int *)&s_dead) refill();
   store_read();
+  cp_async_wait_all();
+  __syncthreads();
+  if (s_dead && threadIdx.x < NS) drain(&full[threadIdx.x], s_pos[threadIdx.x], NS);
 }
 
 // ------------------------------------------------------------- wide pass --
@@ -575,7 +593,10 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1)
   }
   if (threadIdx.x == 0) {
     s_dead = 0;
-    for (int s = 0; s < NS; ++s) slot_init(&full[s]);
+    for (int s = 0; s < NS; ++s) {
+      s_pos[s] = -1;
+      slot_init(&full[s]);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   const WordSize ws(a.lim, (int)a.qn);
@@ -645,10 +666,11 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1)
     if (k == kNotYet) {
       sync();
       if (idx == TU - 1)
-        s_go[g] = slot_wait(&full[slot], parity, &s_pos[slot], pos, a.st, &s_dead) ? unit_of[slot] : -1;
+        s_go[g] = slot_wait(&full[slot], parity, &s_pos[slot], pos, a.st, &s_dead, a.wait) ? unit_of[slot] : kGaveUp;
       sync();
       k = s_go[g];
     }
+    if (k == kGaveUp) break;
     if (k == -1) {
       // no more: pass that on to the group that takes this slot next
       if (idx == 0) {
@@ -663,7 +685,7 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1)
     unsigned next = 0;
     if (idx == 0) next = atomicAdd(&a.st->pipe_ticket, 1u);
     auto done = [&] {  // after a barrier since the last refill()
-      if (idx == 0) s_next[g] = (int)min(next, 0x7fffffffu);
+      if (idx == 0) s_next[g] = *(volatile int *)&s_dead ? 0x7fffffff : (int)min(next, 0x7fffffffu);  // (no ticket: no fill)
       fence_async_smem();
       if (idx == TU - 1) {
         const int np = pos + NG, ns = np % NS;
@@ -744,7 +766,7 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1)
         take_carries<16>(cin, [&](int r) {
           const int m1 = t + r * TR;
           return in + (u == 0 ? (m1 == 0 ? W - 1 : m1 - 1) : m1);
-        }, a.st);
+        }, a.st, a.wait);
       }
       const double W0 = rcn.w0 * cw.x * (w0 ? 0.5 : 1.0), W1 = rcn.w1 * cw.x * (w1 ? 0.5 : 1.0);
       double2 x[16];
@@ -763,7 +785,7 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1)
 #pragma unroll
       for (int r = 0; r < 16; ++r) cell(smb, cells.base + (uint32_t)(t + r * TR) * 32) = x[slot16(r)];
     }
-    if (!extra && tail && idx == 0) await_extra(&a.flags[u == units - 1 ? 0 : u / len + 1], a.st, &s_dead);
+    if (!extra && tail && idx == 0) await_extra(&a.flags[u == units - 1 ? 0 : u / len + 1], a.st, &s_dead, a.wait);
     done();
     if (!extra && lane == 0) {
       store_tile(&map, 4 * u, warp * 256, smb + slot * P::SLOT + warp * 8192);
@@ -773,6 +795,7 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1)
   if (lane == 0) store_read();
   rd.publish(a.st, seen);
   __syncthreads();
+  if (s_dead && threadIdx.x < NS) drain(&full[threadIdx.x], s_pos[threadIdx.x], NS);
   if (threadIdx.x == 0) {
     // the last CTA to leave puts the ticket counter back
     __threadfence();

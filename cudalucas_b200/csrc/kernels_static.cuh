@@ -803,10 +803,10 @@ __device__ __forceinline__ double peek_carry(const double *slot) {
   return c;
 }
 constexpr long long kWaitCycles = 2000000000;  // about a second
-// Takes R carries, slots at(r); the wait is bounded: on expiry it sets the
-// timeout fault bit and goes on.
+// Takes R carries, slots at(r); the wait is bounded (limit, in cycles): on
+// expiry it sets the timeout fault bit and goes on.
 template <int R, class AT>
-__device__ __forceinline__ void take_carries(double *c, AT at, DevState *st) {
+__device__ __forceinline__ void take_carries(double *c, AT at, DevState *st, long long limit) {
   long long t0 = 0;
   for (int k = 0;; ++k) {
     bool missing = false;
@@ -817,7 +817,7 @@ __device__ __forceinline__ void take_carries(double *c, AT at, DevState *st) {
     if (!missing) break;
     const long long now = clock64();
     if (k == 0) t0 = now;
-    else if (now - t0 > kWaitCycles || ((k & 1023) == 0 && (*(volatile uint32_t *)&st->fault & 1u))) {
+    if (now - t0 > limit || ((k & 1023) == 1023 && (*(volatile uint32_t *)&st->fault & 1u))) {
       atomicOr(&st->fault, 1u);
       break;
     }
@@ -982,7 +982,7 @@ __device__ __forceinline__ void wide_body(const WideArgs &a, int blk, S sync = S
       take_carries<16>(cin, [&](int r) {
         const int m1 = t + r * TR;
         return in + (g == 0 ? (m1 == 0 ? W - 1 : m1 - 1) : m1);
-      }, a.st);
+      }, a.st, a.wait);
     }
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
@@ -1139,7 +1139,7 @@ __device__ __forceinline__ void wide_any_body(const WideArgs &a, int blk, S sync
       take_carries<R>(cin, [&](int r) {
         const int m1 = t + r * TR;
         return in + (g == 0 ? (m1 == 0 ? W - 1 : m1 - 1) : m1);
-      }, a.st);
+      }, a.st, a.wait);
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {

@@ -112,6 +112,10 @@ class LLContext:
     def debug_launch(self, which):
         self._check(native.lib().ll_debug_launch(self._h, int(which)), "ll_debug_launch")
 
+    def wait_limit(self, cycles=0):
+        """Limit of the waits inside a pass (0: the built-in one); test hook."""
+        self._check(native.lib().ll_debug_wait_limit(self._h, int(cycles)), "ll_debug_wait_limit")
+
     def inject_failure(self, count=1):
         native.lib().ll_debug_inject_failure(self._h, int(count))
 

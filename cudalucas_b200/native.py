@@ -73,6 +73,7 @@ def lib():
         "ll_check_tables": (i32, []),
         "ll_status_string": (ctypes.c_char_p, [i32]),
         "ll_debug_inject_failure": (None, [vp, i32]),
+        "ll_debug_wait_limit": (i32, [vp, ctypes.c_int64]),
         "ll_debug_launch": (i32, [vp, i32]),
         "ll_step_static": (i32, [ctypes.c_int, u32, u32, u32, u32, vp, vp, fp, vp]),
         "ll_batch_create": (i32, [ctypes.c_int, i32, u32p, u32p, i32, ctypes.POINTER(vp)]),

@@ -167,6 +167,13 @@ const char *ll_status_string(ll_status s);
  * ll_step calls return LL_ERR_INJECTED without touching the device. */
 void ll_debug_inject_failure(ll_ctx *ctx, int32_t count);
 
+/* Test hook: the limit, in SM cycles, of the waits inside a pass of the
+ * specialised kernels (for carries, for slots of the persistent passes).  0:
+ * the built-in limit of about a second; negative: a wait that is not satisfied
+ * at its first look has run out (the next ll_step then returns LL_ERR_TIMEOUT).
+ * Waits for the context's queued work. */
+ll_status ll_debug_wait_limit(ll_ctx *ctx, int64_t cycles);
+
 /* Launches only the tall pass (square) or only the wide pass (carry) of one
  * iteration; used to time and profile the passes separately. */
 ll_status ll_debug_launch(ll_ctx *ctx, int32_t which);
