@@ -1064,6 +1064,7 @@ struct ll_ctx {
   bool ck_valid = false;
   long long *carry = nullptr;
   uint32_t *flags = nullptr;
+  size_t carry_bytes = 0, flag_bytes = 0;
   DevState *st = nullptr;
   DevState *host_st = nullptr;  // pinned copy for the read-back of a step
   double2 *twW = nullptr, *twH = nullptr, *thi = nullptr, *tlo = nullptr;
@@ -1317,10 +1318,11 @@ ll_status ll_create(int device, uint32_t q, uint32_t n, const ll_tuning *tuning,
     if (e != cudaSuccess) { rc = cuda_fail(ctx, e, "stream"); break; }
     const int ngroups = s.H / s.G;
     choose_pipe(ctx, tuning);
-    const size_t flag_bytes = sizeof(uint32_t) * (size_t)std::max(ngroups, 64);
+    const size_t flag_bytes = ctx->flag_bytes = sizeof(uint32_t) * (size_t)std::max(ngroups, 64);
     // a row of carries per row group, or per unit of two rows of the
     // persistent pass
-    const size_t carry_bytes = sizeof(long long) * (size_t)std::max(ngroups, ctx->pipe_w ? s.H / 2 : 0) * s.W;
+    const size_t carry_bytes = ctx->carry_bytes =
+        sizeof(long long) * (size_t)std::max(ngroups, ctx->pipe_w ? s.H / 2 : 0) * s.W;
     if ((e = cudaMalloc((void **)&ctx->A, sizeof(double2) * (size_t)ctx->N)) != cudaSuccess ||
         (e = cudaMalloc((void **)&ctx->xint, sizeof(int32_t) * (size_t)n)) != cudaSuccess ||
         (e = cudaMalloc((void **)&ctx->carry, carry_bytes)) != cudaSuccess ||
@@ -1570,14 +1572,37 @@ static ll_status launch_init(ll_ctx *ctx) {
   return LL_OK;
 }
 
-// Enqueues the state of freshly loaded digits: the shift, no roundoff maximum,
-// no fault.  The counters are kept.
+// The state of freshly loaded digits: the shift, no roundoff maximum, no
+// fault.  After a wait that ran out, carries and flags that came too late are
+// still in their slots, and the next iteration would take them for its own:
+// they are emptied, and the counters put back.  One CTA: without such a fault
+// there is nothing to do but the three words.
+static __global__ void __launch_bounds__(1024) load_state(DevState *st, uint32_t offset, unsigned long long *carry,
+                                                          size_t carries, uint32_t *flags, size_t nflags) {
+  const bool stale = st->fault & 1u;
+  __syncthreads();
+  if (stale) {
+    for (size_t i = threadIdx.x; i < carries; i += blockDim.x) carry[i] = kNoCarryByte * 0x0101010101010101ull;
+    for (size_t i = threadIdx.x; i < nflags; i += blockDim.x) flags[i] = 0;
+  }
+  if (threadIdx.x == 0) {
+    if (stale) {
+      st->ticket = 0;
+      st->bar_count = 0;
+      st->pipe_ticket = 0;
+      st->pipe_exit = 0;
+    }
+    st->offset = offset;
+    st->err_bits = 0;
+    st->fault = 0;
+  }
+}
+
+// Enqueues the state of freshly loaded digits.
 static cudaError_t reset_state(ll_ctx *ctx, uint32_t offset) {
-  const uint32_t f[3] = {offset, 0u, 0u};
-  static_assert(offsetof(DevState, err_bits) == offsetof(DevState, offset) + 4 &&
-                    offsetof(DevState, fault) == offsetof(DevState, offset) + 8,
-                "offset, err_bits and fault are contiguous");
-  return cudaMemcpyAsync(&ctx->st->offset, f, sizeof f, cudaMemcpyHostToDevice, ctx->stream);
+  load_state<<<1, 1024, 0, ctx->stream>>>(ctx->st, offset, (unsigned long long *)ctx->carry, ctx->carry_bytes / 8,
+                                          ctx->flags, ctx->flag_bytes / 4);
+  return cudaGetLastError();
 }
 
 ll_status ll_load_digits(ll_ctx *ctx, const int32_t *digits, uint32_t offset) {

@@ -48,3 +48,27 @@ def test_expired_wait_is_reported_and_leaves_the_gpu_usable(W, H):
         with pytest.raises(cl.LLError):
             c.step(1, errchk=True)
     assert _res64(W, H, 70) == want
+
+
+# rows of 4, 8 and 16 elements per thread beside the persistent passes, the
+# generic kernels' neighbours in one context's life
+@pytest.mark.parametrize("W,H", PIPE + [(256, 320), (512, 720), (512, 1024), (1024, 1024), (2048, 1024)])
+def test_digits_loaded_after_an_expired_wait_give_the_right_residue(W, H):
+    """Carries and flags that came after the wait had run out are gone when
+    digits are loaded (from the host, or from the device checkpoint)."""
+    n = 2 * W * H
+    q = exponent_for(n)
+    want = _res64(W, H, 70)
+    with cl.LLContext(q, n, tuning={"width": W}) as c:
+        for _ in range(3):
+            c.start(q // 3)
+            _expire(c)
+            c.start(q // 3)
+            assert c.step(70, report=True) < 0.4
+            assert c.res64() == want
+        c.start(q // 3)
+        c.device_checkpoint()
+        _expire(c)
+        c.device_restore()
+        assert c.step(70, report=True) < 0.4
+        assert c.res64() == want
