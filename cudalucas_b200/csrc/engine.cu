@@ -1230,19 +1230,27 @@ static int carveout_for(const ll_ctx *ctx, int sms, int bw, int bt) {
   return percent <= 68 ? (int)percent : -1;
 }
 
+// The persistent passes of a shape of n words, if it has any.
+static void pipe_kernels(const Shape &s, uint32_t n, const ll_tuning *tuning, const PipeKernel *&w, const PipeKernel *&t) {
+  w = t = nullptr;
+  if (!s.sw || !s.st || (tuning && (tuning->kernels & LL_KERNELS_NO_PIPE))) return;
+  if (s.H % 2 == 0 && s.sw->tr == s.W / 16 && pipe_rows(s.W, n)) w = find_pipe(s.W);
+  if (pipe_columns(s.H, n)) t = find_pipe(s.H);
+  if (t && !t->tall) t = nullptr;
+}
+
 // Whether the plain iterations of a context run the persistent passes.
 static void choose_pipe(ll_ctx *ctx, const ll_tuning *tuning) {
   const Shape &s = ctx->shape;
+  const PipeKernel *w, *t;
+  pipe_kernels(s, ctx->n, tuning, w, t);
   int sms = 0;
-  if (!s.sw || !s.st || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess)
-    return;
-  const PipeKernel *w = s.H % 2 == 0 && s.sw->tr == s.W / 16 && pipe_rows(s.W, ctx->n) ? find_pipe(s.W) : nullptr;
-  const PipeKernel *t = pipe_columns(s.H, ctx->n) ? find_pipe(s.H) : nullptr;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess) return;
   if (w && cudaFuncSetAttribute(w->wide, cudaFuncAttributeMaxDynamicSharedMemorySize, w->smem_wide) == cudaSuccess) {
     ctx->pipe_w = w;
     ctx->pipe_grid_w = std::min(sms, s.H / 2);
   }
-  if (t && t->tall && cudaFuncSetAttribute(t->tall, cudaFuncAttributeMaxDynamicSharedMemorySize, t->smem_tall) == cudaSuccess) {
+  if (t && cudaFuncSetAttribute(t->tall, cudaFuncAttributeMaxDynamicSharedMemorySize, t->smem_tall) == cudaSuccess) {
     ctx->pipe_t = t;
     ctx->pipe_grid_t = std::min(sms, s.W / 2);
   }
@@ -1821,12 +1829,10 @@ uint64_t ll_context_bytes(uint32_t q, uint32_t n, const ll_tuning *tuning) {
   if (s.sw) b += 16 * (uint64_t)s.sw->extra;
   if (s.st) b += 16 * (uint64_t)s.st->tw;
   // the persistent passes' twiddles, row constants and carry rows
-  if (s.sw && s.st) {
-    const PipeKernel *pw = H % 2 == 0 && s.sw->tr == s.W / 16 && pipe_rows(s.W, n) ? find_pipe(s.W) : nullptr;
-    const PipeKernel *pt = pipe_columns(s.H, n) ? find_pipe(s.H) : nullptr;
-    if (pw) b += 16 * (uint64_t)pw->tw + sizeof(RowConst) * H + (H / 2 > ng ? 8 * (H / 2 - ng) * W : 0);
-    if (pt && pt->tall) b += 16 * (uint64_t)pt->tw;
-  }
+  const PipeKernel *pw, *pt;
+  pipe_kernels(s, n, tuning, pw, pt);
+  if (pw) b += 16 * (uint64_t)pw->tw + sizeof(RowConst) * H + (H / 2 > ng ? 8 * (H / 2 - ng) * W : 0);
+  if (pt) b += 16 * (uint64_t)pt->tw;
   // the cluster kernel's stage twiddles, when the length has one (the
   // largest table among its variants)
   uint64_t tw_cluster = 0;
@@ -1916,7 +1922,8 @@ int32_t ll_check_tables(void) {
 
 int32_t ll_kernel_kinds(const ll_ctx *ctx) {
   if (!ctx) return 0;
-  return (ctx->shape.sw ? 1 : 0) | (ctx->shape.st ? 2 : 0) | (ctx->fused ? 4 : 0) | (ctx->cluster ? 8 : 0);
+  return (ctx->shape.sw ? 1 : 0) | (ctx->shape.st ? 2 : 0) | (ctx->fused ? 4 : 0) | (ctx->cluster ? 8 : 0) |
+         (ctx->pipe_w ? 16 : 0) | (ctx->pipe_t ? 32 : 0);
 }
 void ll_debug_inject_failure(ll_ctx *ctx, int32_t count) {
   if (ctx) ctx->inject = count;

@@ -135,6 +135,7 @@ class LLContext:
         k = native.lib().ll_kernel_kinds(self._h)
         d["wide_specialised"], d["tall_specialised"], d["fused"] = bool(k & 1), bool(k & 2), bool(k & 4)
         d["cluster"] = bool(k & 8)
+        d["wide_persistent"], d["tall_persistent"] = bool(k & 16), bool(k & 32)
         return d
 
 

@@ -81,6 +81,7 @@ typedef struct {
                                      (rows in shared memory, 8 elements per thread);
                                      with any of these flags short lengths run the
                                      rows of 16 elements per thread */
+#define LL_KERNELS_NO_PIPE 64     /* no persistent passes: a launch per unit at long lengths too */
 
 /* Creates a context for exponent q at FFT length n (FP64 words) on `device`.
  * With tuning NULL (or all zero) the engine chooses the launch: for some
@@ -152,7 +153,9 @@ const char *ll_last_error(const ll_ctx *ctx); /* text of the last failure   */
  * pass, bit 1 the tall (column) pass (the others use the generic kernels);
  * bit 2: plain iterations run as fused cooperative launches; bit 3: steps
  * run as cluster-resident launches (the state in the shared memory of one
- * thread-block cluster; from 32K on the steps of fewer than 8 iterations). */
+ * thread-block cluster; from 32K on the steps of fewer than 8 iterations);
+ * bit 4: plain iterations run the persistent row pass, bit 5: the persistent
+ * column pass (one CTA per SM for the whole pass; long lengths). */
 int32_t ll_kernel_kinds(const ll_ctx *ctx);
 /* Host-only self-check of the compiled kernel tables: the number of
  * specialised kernels whose stage-twiddle table (built on the host from the

@@ -70,3 +70,52 @@ def test_opt_in_rows(W, H):
     b = _run(q, n, digits, offset, 70, {"width": W, "kernels": NO_CLUSTER | 32})
     assert a[1] == b[1] and np.array_equal(a[0], b[0])
     assert b[2] < 0.4 and b[2] <= 2 * a[2] + 1e-3 and a[2] <= 2 * b[2] + 1e-3
+
+
+NO_PIPE = 64
+ROWS = {1024, 1280, 1536, 1792, 2048, 2304, 2560, 3072, 3584, 4096}
+
+
+# both sides of the lines: 3000K and 9000K (rows of 1792) for rows, columns of
+# 1280 and 2304K for columns; rows of 768 and columns of other lengths never
+@pytest.mark.parametrize("W,H,rows,columns", [
+    (1024, 1024, False, False), (1024, 1568, True, False), (2560, 576, False, False), (3072, 576, True, False),
+    (1792, 1792, False, True), (1792, 2688, True, False), (768, 3072, False, True), (2048, 1024, True, False),
+    (512, 2048, False, False), (512, 2304, False, True), (1280, 1280, True, True), (4096, 4096, True, True)])
+def test_persistent_passes_run_where_the_rule_says(W, H, rows, columns):
+    n = 2 * W * H
+    q = exponent_for(n)
+    with cl.LLContext(q, n, tuning={"width": W}) as c:
+        assert (c.shape["wide_persistent"], c.shape["tall_persistent"]) == (rows, columns)
+    with cl.LLContext(q, n, tuning={"width": W, "kernels": NO_PIPE}) as c:
+        assert c.shape["W"] == W and not c.shape["wide_persistent"] and not c.shape["tall_persistent"]
+
+
+@pytest.mark.parametrize("W,H", [(1024, 1568), (1280, 1280), (1536, 1536), (1792, 2688), (2048, 2048), (2304, 2304),
+                                 (2560, 1280), (3072, 1536), (3584, 1792), (4096, 392), (512, 2304), (512, 3584)])
+def test_persistent_passes_equal_a_launch_per_unit(W, H):
+    """Same shape, same carry arithmetic: the digits are the same bit for bit;
+    and the residue after a few iterations is the oracle's."""
+    from oracle.binding import Oracle, set_threads
+    n = 2 * W * H
+    q = exponent_for(n)
+    digits, offset = _random_digits(q, n, W + H)
+    d, o, err, _ = _run(q, n, digits, offset, 130, {"width": W})
+    g, go, gerr, _ = _run(q, n, digits, offset, 130, {"width": W, "kernels": NO_PIPE})
+    assert o == go and np.array_equal(d, g)
+    assert err <= 2 * gerr + 1e-3 and gerr <= 2 * err + 1e-3, (err, gerr)
+    if n > 3 << 20:
+        return
+    with cl.LLContext(q, n, tuning={"width": W}) as c:
+        c.start(q // 5)
+        c.step(6)
+        c.step(2, report=True)
+        got = c.res64()
+    set_threads(16)
+    try:
+        ref = Oracle(q, n)
+        ref.start(q // 5)
+        ref.step(8)
+        assert got == ref.res64()
+    finally:
+        set_threads(1)
