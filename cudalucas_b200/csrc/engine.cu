@@ -742,9 +742,9 @@ using namespace llb;
 
 namespace {
 
-// e^{2 pi i num/den} rounded once from 80-bit arithmetic, with the angle
-// reduced to the first octant so that cosl/sinl see small arguments.
-double2 unit_root(unsigned long long num, unsigned long long den) {
+// e^{2 pi i num/den} from 80-bit arithmetic, with the angle reduced to the
+// first octant so that cosl/sinl see small arguments.
+void unit_root_l(unsigned long long num, unsigned long long den, long double &c, long double &s) {
   num %= den;
   // angle fraction f = num/den in [0,1); use 8*num relative to den for octant
   const long double PI = 3.14159265358979323846264338327950288L;
@@ -752,7 +752,6 @@ double2 unit_root(unsigned long long num, unsigned long long den) {
   int oct = (int)(n8 / den);
   long double rem = (long double)(n8 - (unsigned long long)oct * den) / (long double)den;  // [0,1)
   long double a = rem * PI / 4;  // [0, pi/4)
-  long double c, s;
   long double ca = cosl(a), sa = sinl(a), cb = cosl(PI / 4 - a), sb = sinl(PI / 4 - a);
   switch (oct) {
     case 0: c = ca; s = sa; break;
@@ -764,6 +763,11 @@ double2 unit_root(unsigned long long num, unsigned long long den) {
     case 6: c = sa; s = -ca; break;
     default: c = cb; s = -sb; break;
   }
+}
+// The same, rounded once.
+double2 unit_root(unsigned long long num, unsigned long long den) {
+  long double c, s;
+  unit_root_l(num, den, c, s);
   return make_double2((double)c, (double)s);
 }
 
@@ -947,14 +951,54 @@ std::vector<double2> stage_twiddles(const int *rad, int nrad) {
 
 }  // namespace
 
-// tan(2*pi*num/den), from the nearer end of the quarter turn.
-static double tangent(unsigned long long num, unsigned long long den) {
-  const long double PI = 3.14159265358979323846264338327950288L;
-  const unsigned long long n4 = num % den * 4, quarter = n4 / den, rem = n4 - quarter * den;
-  const bool upper = 2 * rem > den;
-  long double t = tanl((long double)(upper ? den - rem : rem) / (long double)den * (PI / 2));
-  if (upper) t = 1 / t;
-  return (double)(quarter & 1 ? -1 / t : t);
+// Cosine and tangent of 2*pi*num/den as the persistent passes' butterflies take
+// them (twiddle c + i*c*t): of the neighbouring values the pair whose twiddle is
+// nearest to one of length 1 + bias.
+static double2 cos_tan(unsigned long long num, unsigned long long den, long double bias) {
+  if (4 * (num % den) == den) return make_double2(0x1p-60, 0x1p60);  // a cosine far below rounding keeps the tangent finite
+  long double x, y;
+  unit_root_l(num, den, x, y);
+  const double c0 = (double)x, t0 = (double)(y / x);
+  if (t0 == 0.0) return make_double2(c0, t0);
+  x += bias * x;
+  y += bias * y;
+  double2 best = make_double2(c0, t0);
+  long double least = 1.0L;
+  double c = nextafter(c0, -INFINITY);
+  for (int i = 0; i < 3; ++i, c = nextafter(c, INFINITY)) {
+    double t = nextafter(nextafter(t0, -INFINITY), -INFINITY);
+    for (int j = 0; j < 5; ++j, t = nextafter(t, INFINITY)) {
+      const long double ex = (long double)c - x, ey = (long double)c * (long double)t - y, e = ex * ex + ey * ey;
+      if (e < least) {
+        least = e;
+        best = make_double2(c, t);
+      }
+    }
+  }
+  return best;
+}
+
+// The bias of a length 256*M, in units of 2^-53.  A transform whose constants and
+// twiddles are rounded to 53 bits has a gain other than one: the register
+// transforms of 16 and M points by their constants alone (16 points 0.126, 6, 9 and
+// 12 points -0.30, -0.38 and -0.30 of those units, from sin(pi/3) and sqrt(1/2)), the
+// stage-1 twiddles by their mean.  The eight entries have a weight of two in all;
+// with this bias the transform's gain, computed exactly from the constants and
+// the table, is below 0.01 units (by bisection).
+static double twiddle_bias(int M) {
+  switch (M) {
+    case 4: return -0.1054;
+    case 5: return -0.0944;
+    case 6: return 0.1276;
+    case 7: return -0.0858;
+    case 8: return -0.1921;
+    case 9: return 0.1510;
+    case 10: return -0.0574;
+    case 12: return 0.1167;
+    case 14: return -0.0696;
+    case 16: return -0.1654;
+  }
+  return 0.0;
 }
 
 // Twiddle table of the persistent passes for length L = 256*M (see
@@ -963,14 +1007,12 @@ static double tangent(unsigned long long num, unsigned long long den) {
 static std::vector<double2> pipe_twiddles(int L) {
   const int M = L / 256, TR = L / 16, SS = M | 1;
   std::vector<double2> out((size_t)8 * TR + (M > 1 ? 16 * SS : 0), make_double2(0.0, 0.0));
-  static const int power[8] = {8, 4, 2, 2, 1, 1, 1, 1}, root[8] = {0, 0, 0, 2, 0, 1, 2, 3};
+  // sixteenths of a turn: entries 3, 6 and 7 (w8, w8, w16^3) a quarter back
+  static const int power[8] = {8, 4, 2, 2, 1, 1, 1, 1}, root[8] = {0, 0, 0, 2 - 4, 0, 1, 2 - 4, 3 - 4};
+  const long double bias = (long double)twiddle_bias(M) * 0x1p-53L;
   for (int c = 0; c < TR; ++c)
-    for (int e = 0; e < 8; ++e) {
-      const int num = power[e] * c + root[e] * (L / 16);  // less than half a turn
-      // the quarter turn: a cosine far below rounding keeps the tangent finite
-      out[(size_t)e * TR + c] = 4 * num == L ? make_double2(0x1p-60, 0x1p60)
-                                             : make_double2(unit_root(num, L).x, tangent(num, L));
-    }
+    for (int e = 0; e < 8; ++e)
+      out[(size_t)e * TR + c] = cos_tan((unsigned long long)(L + power[e] * c + root[e] * (L / 16)), L, bias);
   if (M > 1)
     for (int j = 0; j < 16; ++j)
       for (int v = 0; v < M; ++v) out[(size_t)8 * TR + j * SS + v] = unit_root((unsigned long long)j * v, TR);

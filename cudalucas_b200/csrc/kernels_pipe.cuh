@@ -53,25 +53,39 @@ struct Pipe {
 
 // Twiddle table of a length: entry e < 8 of thread c at [e*TR + c], cosine and
 // tangent of the powers of z = w_L^c that dft16_tw takes: z^8, z^4, z^2,
-// z^2*w8, z, z*w16, z*w8, z*w16^3; then the stage-1 twiddles w_TR^(j0*v) at [8*TR + j0*SS + v].
+// -i*z^2*w8, z, z*w16, -i*z*w8, -i*z*w16^3; then the stage-1 twiddles w_TR^(j0*v) at
+// [8*TR + j0*SS + v].
 
 // a + e*b and a - e*b in six fused operations; w.x is the cosine, w.y the
 // tangent of the twiddle: e*b = c*(b + i*t*b), so each result has two
-// roundings.  (With a - e*b as 2a - (a + e*b) it has three: a transform of 3072
-// then has an rms error of 2.08 units, this 1.99, products and dft16 1.97.)
-// e = w, or i*w with ROT; conjugated for SIGN < 0.
-template <int SIGN, bool ROT>
+// roundings.  (With a - e*b as 2a - (a + e*b) it has three.)  e = i^Q * w,
+// conjugated for SIGN < 0.
+//
+// Accuracy.  An error of the stored cosine scales both parts of the twiddle, so
+// with cosine and tangent rounded each by itself the twiddle's own error has up
+// to twice the variance of a rounded (cosine, sine) pair.  And what the errors of
+// all twiddles and constants have in common, a gain of the whole transform, adds
+// up over the two passes: at 3072 x 3072 the rms of all roundoffs was 0.02111,
+// with products and dft16 0.02031.  So the table holds the pair of neighbouring
+// values whose twiddle has the smallest error, entries 3, 6 and 7 are turned back
+// by a quarter (tangents below one), and the twiddles aim at a length that
+// cancels the gain (host side).  Squaring of random words by two transforms of
+// length L, rms error in units of 2^-53 and the gain of the square, products /
+// rounded singly / this: 2304 3.52, -0.4 / 3.68, -0.7 / 3.43, 0.0; 3072 3.43, -0.2 /
+// 3.53, -0.5 / 3.37, 0.0; 4096 3.72, 1.3 / 3.73, 1.2 / 3.41, 0.0; the other lengths 2
+// to 9 % below products too.
+template <int SIGN, int Q>
 __device__ __forceinline__ void bfly(double2 &a, double2 &b, double2 w) {
-  const double c = w.x, t = SIGN > 0 ? w.y : -w.y;
-  const double ux = fma(-t, b.y, b.x), uy = fma(t, b.x, b.y);  // w*b = c*u
-  const double rx = ROT ? (SIGN > 0 ? -uy : uy) : ux, ry = ROT ? (SIGN > 0 ? ux : -ux) : uy;
+  const double c = Q & 2 ? -w.x : w.x, t = SIGN > 0 ? w.y : -w.y;
+  const double ux = fma(-t, b.y, b.x), uy = fma(t, b.x, b.y);  // w*b = c*u, up to the sign of Q & 2
+  const double rx = Q & 1 ? (SIGN > 0 ? -uy : uy) : ux, ry = Q & 1 ? (SIGN > 0 ? ux : -ux) : uy;
   b = make_double2(fma(-c, rx, a.x), fma(-c, ry, a.y));
   a = make_double2(fma(c, rx, a.x), fma(c, ry, a.y));
 }
 
 // 16-point DFT of v[r]*z^r in 192 fused operations (60 of complex products
 // and 160 of dft16 before): radix-2 layers whose twiddles are powers of z
-// times sixteenth roots, 8 different up to a factor i.  tw(e) gives entry e
+// times sixteenth roots, 8 different up to a power of i.  tw(e) gives entry e
 // of the table above.  Output k is left in v[slot16(k)].
 __device__ __forceinline__ constexpr int slot16(int k) {  // bit reversal
   return ((k & 1) << 3) | ((k & 2) << 1) | ((k & 4) >> 1) | ((k & 8) >> 3);
@@ -81,35 +95,35 @@ __device__ __forceinline__ void dft16_tw(double2 *v, TW tw) {
   {
     const double2 w = tw(0);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) bfly<SIGN, false>(v[j], v[j + 8], w);
+    for (int j = 0; j < 8; ++j) bfly<SIGN, 0>(v[j], v[j + 8], w);
   }
   {
     const double2 w = tw(1);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      bfly<SIGN, false>(v[j], v[j + 4], w);
-      bfly<SIGN, true>(v[8 + j], v[8 + j + 4], w);
+      bfly<SIGN, 0>(v[j], v[j + 4], w);
+      bfly<SIGN, 1>(v[8 + j], v[8 + j + 4], w);
     }
   }
   {
     const double2 w = tw(2), w8 = tw(3);
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      bfly<SIGN, false>(v[j], v[j + 2], w);
-      bfly<SIGN, true>(v[4 + j], v[4 + j + 2], w);
-      bfly<SIGN, false>(v[8 + j], v[8 + j + 2], w8);
-      bfly<SIGN, true>(v[12 + j], v[12 + j + 2], w8);
+      bfly<SIGN, 0>(v[j], v[j + 2], w);
+      bfly<SIGN, 1>(v[4 + j], v[4 + j + 2], w);
+      bfly<SIGN, 1>(v[8 + j], v[8 + j + 2], w8);
+      bfly<SIGN, 2>(v[12 + j], v[12 + j + 2], w8);
     }
   }
   // nodes k mod 8 = 0, 4 (rotated), 2, 6, 1, 5, 3, 7
-  bfly<SIGN, false>(v[0], v[1], tw(4));
-  bfly<SIGN, true>(v[2], v[3], tw(4));
-  bfly<SIGN, false>(v[4], v[5], tw(6));
-  bfly<SIGN, true>(v[6], v[7], tw(6));
-  bfly<SIGN, false>(v[8], v[9], tw(5));
-  bfly<SIGN, true>(v[10], v[11], tw(5));
-  bfly<SIGN, false>(v[12], v[13], tw(7));
-  bfly<SIGN, true>(v[14], v[15], tw(7));
+  bfly<SIGN, 0>(v[0], v[1], tw(4));
+  bfly<SIGN, 1>(v[2], v[3], tw(4));
+  bfly<SIGN, 1>(v[4], v[5], tw(6));
+  bfly<SIGN, 2>(v[6], v[7], tw(6));
+  bfly<SIGN, 0>(v[8], v[9], tw(5));
+  bfly<SIGN, 1>(v[10], v[11], tw(5));
+  bfly<SIGN, 1>(v[12], v[13], tw(7));
+  bfly<SIGN, 2>(v[14], v[15], tw(7));
 }
 
 // e^(2 pi i e/16), e a compile-time value after unrolling.

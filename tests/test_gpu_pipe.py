@@ -119,3 +119,21 @@ def test_persistent_passes_equal_a_launch_per_unit(W, H):
         assert got == ref.res64()
     finally:
         set_threads(1)
+
+
+@pytest.mark.parametrize("W,H", [(2304, 2304), (3072, 2304), (3072, 3072), (1792, 2688), (4096, 2304), (1536, 1536),
+                                 (3584, 3584)])
+def test_persistent_passes_are_as_accurate_as_a_launch_per_unit(W, H):
+    """Mean over 200 iterations of the largest roundoff, same digits on both
+    sides.  A single maximum scatters by about 8 %, so the means by 0.6 % each:
+    3 % is more than three times the scatter of their ratio."""
+    n = 2 * W * H
+    q = exponent_for(n)
+    mean = []
+    for kernels in (0, NO_PIPE):
+        with cl.LLContext(q, n, tuning={"width": W, "kernels": kernels}) as c:
+            assert c.shape["wide_persistent"] == (kernels == 0)
+            c.start(q // 3)
+            c.step(64, errchk=True)
+            mean.append(sum(c.step(1, errchk=True) for _ in range(200)) / 200)
+    assert mean[0] <= 1.03 * mean[1], mean
