@@ -547,20 +547,29 @@ static const StaticWide kWide[] = {
     LLB_WIDE_ANY(F768, 2, 2, kAltRows),
     LLB_WIDE_ANY(F1024, 2, 2, kAltRows), LLB_WIDE_ANY(F1280, 2, 3, kAltRows),
 };
+static bool has_fused(long long W, long long H);
 // The row kernel variants a context of N = L*H may use: with
 // LL_KERNELS_ALT_WIDE the alternative kernel of a length replaces the others
 // of that length; for few row groups the short one does, unless the caller
-// chooses kernels (then 16 elements per thread, as the fused kernels have).
+// asks for 16 elements per thread (LL_KERNELS_LONG_ROWS).  Shapes with a fused
+// kernel keep to its rows, of 16 elements, where the caller asks for it or for
+// two launches in its place.
 static bool short_rows(const StaticWide &k, long long N, const ll_tuning *t) {
-  return k.alt == kShortRows && N / k.L / k.G <= kShortGroups && !(t && t->kernels);
+  if (k.alt != kShortRows || N / k.L / k.G > kShortGroups) return false;
+  const int32_t f = t ? t->kernels : 0;
+  if (f & LL_KERNELS_LONG_ROWS) return false;
+  return !((f & (LL_KERNELS_FUSED | LL_KERNELS_NO_CLUSTER)) && has_fused(k.L, N / k.L));
 }
 static bool wide_allowed(const StaticWide &w, long long N, const ll_tuning *t) {
   const bool want_alt = t && (t->kernels & LL_KERNELS_ALT_WIDE);
-  if (w.alt == kShortRows) return short_rows(w, N, t);
-  if (w.alt) return want_alt;
+  if (w.alt == kAltRows) return want_alt;
+  bool alt = false, few = false;
   for (const auto &k : kWide)
-    if (k.L == w.L && ((k.alt == kAltRows && want_alt) || short_rows(k, N, t))) return false;
-  return true;
+    if (k.L == w.L) {
+      alt |= k.alt == kAltRows && want_alt;
+      few |= short_rows(k, N, t);
+    }
+  return !alt && (w.alt == kShortRows) == few;
 }
 // Column lengths outside the 16 x M x 16 family that the length policy meets
 // with a specialised row length: the fewest stages of radices <= 16, and the
@@ -632,6 +641,11 @@ static const FusedKernel kFused[] = {
     LLB_FUSED(L256, 2, C28, 7, 16),
     LLB_FUSED(L256, 2, C112, 8, 4),
 };
+static bool has_fused(long long W, long long H) {
+  for (const auto &k : kFused)
+    if (k.W == W && k.H == H) return true;
+  return false;
+}
 static const FusedKernel *find_fused(int W, int H, int G) {
   for (const auto &k : kFused)
     if (k.W == W && k.H == H && k.G == G) return &k;
@@ -2388,7 +2402,7 @@ ll_status ll_batch_create(int device, int32_t count, const uint32_t *q, const ui
   // of a pass: it takes the 16-element rows nearest sqrt(N) rather than what is
   // fastest alone (32 members of 50K to 1024K, 390 iterations: 91.6 ms with the
   // solo choice, 81.4 with this).
-  t.kernels = LL_KERNELS_NO_CLUSTER;
+  t.kernels = LL_KERNELS_NO_CLUSTER | LL_KERNELS_LONG_ROWS;
   for (int32_t i = 0; i < count; ++i) {
     ll_ctx *c = nullptr;
     ll_status s = ll_create(device, q[i], n[i], &t, &c);

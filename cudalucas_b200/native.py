@@ -28,6 +28,7 @@ LL_KERNELS_NO_CLUSTER = 8
 LL_KERNELS_CLUSTER8 = 16
 LL_KERNELS_ALT_WIDE = 32
 LL_KERNELS_NO_PIPE = 64
+LL_KERNELS_LONG_ROWS = 128
 
 
 class Tuning(ctypes.Structure):

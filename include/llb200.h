@@ -70,7 +70,8 @@ typedef struct {
  * 16K, 18K, 20K; 32K, 36K, 42K, 48K, 56K for steps of fewer than 8 iterations)
  * run an ll_step as one launch of one thread-block cluster whose shared memory
  * holds the whole state;
- * LL_KERNELS_NO_CLUSTER turns that off (two launches per iteration),
+ * LL_KERNELS_NO_CLUSTER turns that off (two launches per iteration; at 12K,
+ * 14K and 56K with the rows of the fused kernel, 16 elements per thread),
  * LL_KERNELS_CLUSTER8 keeps to the portable cluster size of 8 CTAs. */
 #define LL_KERNELS_GENERIC 1
 #define LL_KERNELS_FUSED 2
@@ -78,9 +79,9 @@ typedef struct {
 #define LL_KERNELS_NO_CLUSTER 8   /* no cluster-resident iterations */
 #define LL_KERNELS_CLUSTER8 16    /* clusters of at most 8 CTAs */
 #define LL_KERNELS_ALT_WIDE 32    /* the alternative row kernel where a length has one
-                                     (rows in shared memory, 8 elements per thread);
-                                     with any of these flags short lengths run the
-                                     rows of 16 elements per thread */
+                                     (rows in shared memory, 8 elements per thread) */
+#define LL_KERNELS_LONG_ROWS 128  /* rows of 16 elements per thread at short lengths too (rows of
+                                     256 and 512 have 4 and 8 for passes of few rows) */
 #define LL_KERNELS_NO_PIPE 64     /* no persistent passes: a launch per unit at long lengths too */
 
 /* Creates a context for exponent q at FFT length n (FP64 words) on `device`.
@@ -187,8 +188,8 @@ ll_status ll_debug_launch(ll_ctx *ctx, int32_t which);
  * ll_read_digits, ...); one step of `graph_iters` iterations of all members is
  * replayed from a single CUDA graph in which every member is a parallel
  * branch, so members of different lengths overlap on the GPU.  A member runs
- * the kernels of a solo run with LL_KERNELS_NO_CLUSTER: its residues equal the
- * solo residues. */
+ * the kernels of a solo run with LL_KERNELS_NO_CLUSTER and
+ * LL_KERNELS_LONG_ROWS: its residues equal the solo residues. */
 typedef struct ll_batch ll_batch;
 ll_status ll_batch_create(int device, int32_t count, const uint32_t *q, const uint32_t *n, int32_t graph_iters,
                           ll_batch **out);
