@@ -1602,32 +1602,35 @@ static void launch_static(const void *k, void *args, int grid, int threads, size
   cudaLaunchKernelExC(&cfg, k, argv);
 }
 
-static void launch_wide(ll_ctx *ctx, int mode, bool chained = false) {
+// (`on`: another stream than the context's own)
+static void launch_wide(ll_ctx *ctx, int mode, bool chained = false, cudaStream_t on = nullptr) {
   const Shape &s = ctx->shape;
+  const cudaStream_t st = on ? on : ctx->stream;
   const size_t sm = shape_wide_smem(s);
   if (ctx->pipe_w && mode == WIDE_ITER) {
     const PipeKernel *p = ctx->pipe_w;
-    launch_static((const void *)p->wide, &ctx->wa, ctx->pipe_grid_w, p->threads, p->smem_wide, ctx->stream, chained,
+    launch_static((const void *)p->wide, &ctx->wa, ctx->pipe_grid_w, p->threads, p->smem_wide, st, chained,
                   ctx->carveout, &ctx->map);
   } else if (s.sw) {
     void (*k)(WideArgs) = mode == WIDE_INIT ? s.sw->init : mode == WIDE_REPORT ? s.sw->report : s.sw->iter;
-    launch_static((const void *)k, &ctx->wa, s.H / s.G, s.T1, sm, ctx->stream, chained && ctx->pdl, ctx->carveout);
+    launch_static((const void *)k, &ctx->wa, s.H / s.G, s.T1, sm, st, chained && ctx->pdl, ctx->carveout);
   } else if (mode == WIDE_INIT) {
-    wide_kernel<EPT, WIDE_INIT><<<s.H / s.G, s.T1, sm, ctx->stream>>>(ctx->wa);
+    wide_kernel<EPT, WIDE_INIT><<<s.H / s.G, s.T1, sm, st>>>(ctx->wa);
   } else if (mode == WIDE_REPORT) {
-    wide_kernel<EPT, WIDE_REPORT><<<s.H / s.G, s.T1, sm, ctx->stream>>>(ctx->wa);
+    wide_kernel<EPT, WIDE_REPORT><<<s.H / s.G, s.T1, sm, st>>>(ctx->wa);
   } else {
     wide_kernel<EPT, WIDE_ITER><<<s.H / s.G, s.T1, sm, ctx->stream>>>(ctx->wa);
   }
 }
 
-static void launch_tall(ll_ctx *ctx, bool chained = false) {
+static void launch_tall(ll_ctx *ctx, bool chained = false, cudaStream_t on = nullptr) {
   const Shape &s = ctx->shape;
+  const cudaStream_t st = on ? on : ctx->stream;
   if (ctx->pipe_t) {
     const PipeKernel *p = ctx->pipe_t;
-    launch_static((const void *)p->tall, &ctx->ta, ctx->pipe_grid_t, p->threads, p->smem_tall, ctx->stream, chained, ctx->carveout);
-  } else if (s.st) launch_static((const void *)s.st->run, &ctx->ta, tall_grid(s), s.T2, shape_tall_smem(s), ctx->stream, chained && ctx->pdl, ctx->carveout);
-  else tall_kernel<EPT><<<s.W / 2, s.T2, tall_smem(s.H), ctx->stream>>>(ctx->ta);
+    launch_static((const void *)p->tall, &ctx->ta, ctx->pipe_grid_t, p->threads, p->smem_tall, st, chained, ctx->carveout);
+  } else if (s.st) launch_static((const void *)s.st->run, &ctx->ta, tall_grid(s), s.T2, shape_tall_smem(s), st, chained && ctx->pdl, ctx->carveout);
+  else tall_kernel<EPT><<<s.W / 2, s.T2, tall_smem(s.H), st>>>(ctx->ta);
 }
 
 static ll_status launch_init(ll_ctx *ctx) {
@@ -2276,6 +2279,11 @@ extern "C" ll_status ll_step_static(int device, uint32_t q, uint32_t n, uint32_t
 // Members of one FFT length whose passes both have specialised kernels run
 // as a length class: one launch per pass for all of them (blockIdx.x =
 // member * units + unit), the members' kernel arguments in a device array.
+// Members with persistent passes follow one another on one branch: a pass of
+// theirs has a CTA on every SM, and two at a time take the SMs from each other
+// (us per iteration of all members, as a class / side by side / in turn: 2 of
+// 3200K 115 / 120 / 110, 2 of 8064K 356 / 315 / 276, 4 of 8064K 685 / 635 / 552, 2 of
+// 14336K 680 / 442 / 478, 2 of 18432K 720 / 594 / 548).
 struct BatchClass {
   std::vector<int> idx;  // members
   const StaticTall *st = nullptr;
@@ -2297,6 +2305,7 @@ struct ll_batch {
   bool by_class = true;                 // one launch per pass per length class (else per member)
   std::vector<BatchClass> classes;
   std::vector<int> singles;             // members launched on their own
+  std::vector<int> serial;              // members with persistent passes, one after the other
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
   std::string err;
@@ -2324,6 +2333,10 @@ static ll_status build_classes(ll_batch *b) {
   std::vector<int> order;
   for (size_t i = 0; i < b->members.size(); ++i) {
     const ll_ctx *c = b->members[i];
+    if (c->pipe_w || c->pipe_t) {
+      b->serial.push_back((int)i);
+      continue;
+    }
     if (!(c->shape.sw && c->shape.st && c->shape.st->batch)) {
       b->singles.push_back((int)i);
       continue;
@@ -2387,6 +2400,32 @@ static void launch_class(const void *kern, const void *arr, int units, int count
   cudaLaunchKernelExC(&cfg, kern, argv);
 }
 
+// The launch that a batch's members of n words run, of `total` words in all (us
+// per iteration of all members).  A batch of few words does not fill the GPU:
+// what is fastest alone is fastest (16 members of 50K 27.5 with 16 elements per
+// thread / 19.2 as alone, 2 of 400K 28.2 / 22.2, 2 of 720K 36.0 / 34.4).  Above about
+// 1700K words it is bound by the work of all members, and rows of 16 elements do
+// less of it (16 of 160K 39.2 / 45.3, 4 of 448K 32.5 / 34.4, 8 of 448K 57.8 / 63.2;
+// at 1600K words 16 of 100K 32.2 / 32.0, 1 of 1600K 41.9 / 39.7; single lengths lie
+// on the other side, 2 of 512K 21.1 / 23.9).  There a launch preference still holds
+// if it was measured with such rows (16 of 640K nearest sqrt(N) / preferred 197 /
+// 148, 8 of 896K 132 / 97, 4 of 1296K 119 / 105), not if with short or alternative
+// ones (16 of 1152K 287 / 367, 32 of 160K 70.4 / 73.3).
+constexpr uint64_t kSoloWords = 1700u * 1024;
+static ll_tuning batch_tuning(uint32_t n, uint64_t total) {
+  ll_tuning t{};
+  if (total > kSoloWords) {
+    ll_tuning pref{};
+    const ll_tuning *p = effective_tuning(n, nullptr, pref);
+    Shape s;
+    if (p && choose_shape((long long)n / 2, p, s) && s.sw && s.sw->alt == 0) t = *p;
+    else t.kernels = LL_KERNELS_NO_CLUSTER;
+    t.kernels |= LL_KERNELS_LONG_ROWS;
+  }
+  t.graph_iters = -1;  // members never capture their own graphs
+  return t;
+}
+
 extern "C" {
 
 ll_status ll_batch_create(int device, int32_t count, const uint32_t *q, const uint32_t *n, int32_t graph_iters,
@@ -2396,15 +2435,11 @@ ll_status ll_batch_create(int device, int32_t count, const uint32_t *q, const ui
   ll_batch *b = new ll_batch();
   b->device = device;
   b->graph_iters = graph_iters > 0 ? graph_iters : 10;
-  ll_tuning t{};
-  t.graph_iters = -1;  // members never capture their own graphs
-  // A batch is bound by the work of all members together, not by the latency
-  // of a pass: it takes the 16-element rows nearest sqrt(N) rather than what is
-  // fastest alone (32 members of 50K to 1024K, 390 iterations: 91.6 ms with the
-  // solo choice, 81.4 with this).
-  t.kernels = LL_KERNELS_NO_CLUSTER | LL_KERNELS_LONG_ROWS;
+  uint64_t total = 0;
+  for (int32_t i = 0; i < count; ++i) total += n[i];
   for (int32_t i = 0; i < count; ++i) {
     ll_ctx *c = nullptr;
+    const ll_tuning t = batch_tuning(n[i], total);
     ll_status s = ll_create(device, q[i], n[i], &t, &c);
     if (s != LL_OK) {
       free_batch(b);
@@ -2477,6 +2512,17 @@ ll_status ll_batch_step(ll_batch *b, uint32_t iters, uint32_t flags, float *max_
           cudaStreamWaitEvent(b->stream, b->events[ev++], 0);
         }
         alone = b->singles;
+        if (!b->serial.empty()) {
+          const cudaStream_t on = b->members[(size_t)b->serial[0]]->stream;
+          cudaStreamWaitEvent(on, b->events[0], 0);
+          for (int i : b->serial)
+            for (uint32_t k = 0; k < K; ++k) {
+              launch_tall(b->members[(size_t)i], k > 0, on);
+              launch_wide(b->members[(size_t)i], WIDE_ITER, true, on);
+            }
+          cudaEventRecord(b->events[ev], on);
+          cudaStreamWaitEvent(b->stream, b->events[ev++], 0);
+        }
       } else {
         for (size_t i = 0; i < b->members.size(); ++i) alone.push_back((int)i);
       }

@@ -186,10 +186,13 @@ ll_status ll_debug_launch(ll_ctx *ctx, int32_t which);
  * process): `count` exponents q[i] at lengths n[i] advance together.  Each
  * member is a full context (ll_batch_member gives it for ll_load_digits,
  * ll_read_digits, ...); one step of `graph_iters` iterations of all members is
- * replayed from a single CUDA graph in which every member is a parallel
- * branch, so members of different lengths overlap on the GPU.  A member runs
- * the kernels of a solo run with LL_KERNELS_NO_CLUSTER and
- * LL_KERNELS_LONG_ROWS: its residues equal the solo residues. */
+ * replayed from a single CUDA graph in which every length class (see
+ * ll_batch_group_by_length) is a parallel branch, so members of different
+ * lengths overlap on the GPU; members long enough for the persistent passes,
+ * each of which takes the whole GPU, follow one another on one branch.  The
+ * members' launch is chosen by the words of the whole batch: few, and a member
+ * runs as it would alone (two launches per iteration); many, and rows have 16
+ * elements per thread (LL_KERNELS_LONG_ROWS).  Residues equal solo residues. */
 typedef struct ll_batch ll_batch;
 ll_status ll_batch_create(int device, int32_t count, const uint32_t *q, const uint32_t *n, int32_t graph_iters,
                           ll_batch **out);
