@@ -976,19 +976,24 @@ static double2 cos_tan(unsigned long long num, unsigned long long den, long doub
   if (t0 == 0.0) return make_double2(c0, t0);
   x += bias * x;
   y += bias * y;
+  auto step = [](double v, int places) {  // (v is not zero)
+    int64_t bits;
+    memcpy(&bits, &v, sizeof bits);
+    bits += places;
+    memcpy(&v, &bits, sizeof v);
+    return v;
+  };
   double2 best = make_double2(c0, t0);
   long double least = 1.0L;
-  double c = nextafter(c0, -INFINITY);
-  for (int i = 0; i < 3; ++i, c = nextafter(c, INFINITY)) {
-    double t = nextafter(nextafter(t0, -INFINITY), -INFINITY);
-    for (int j = 0; j < 5; ++j, t = nextafter(t, INFINITY)) {
+  for (int i = -1; i <= 1; ++i)
+    for (int j = -2; j <= 2; ++j) {
+      const double c = step(c0, i), t = step(t0, j);
       const long double ex = (long double)c - x, ey = (long double)c * (long double)t - y, e = ex * ex + ey * ey;
       if (e < least) {
         least = e;
         best = make_double2(c, t);
       }
     }
-  }
   return best;
 }
 
@@ -1122,7 +1127,7 @@ struct ll_ctx {
   uint32_t *flags = nullptr;
   size_t carry_bytes = 0, flag_bytes = 0;
   DevState *st = nullptr;
-  DevState *host_st = nullptr;  // pinned copy for the read-back of a step
+  DevState *host_st = nullptr;  // pinned copy for the read-back of a step (a slot of the status pages)
   double2 *twW = nullptr, *twH = nullptr, *thi = nullptr, *tlo = nullptr;
   double2 *stwW = nullptr, *stwH = nullptr;
   const PipeKernel *pipe_w = nullptr, *pipe_t = nullptr;  // persistent passes of plain iterations
@@ -1173,6 +1178,55 @@ static cudaError_t upload(T **dst, const std::vector<T> &v) {
   return cudaMemcpy(*dst, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice);
 }
 
+// Pinned host memory for the read-backs of all contexts, in pages of slots
+// (pinning 64 bytes for each context took 2.6 of the 3.3 ms in which a context of
+// 12K is made).  A page is given back with its last slot, except for one that is
+// kept for the next context; slots of different devices share pages.
+namespace {
+constexpr size_t kStatusSlot = 64, kStatusSlots = 64;
+static_assert(sizeof(DevState) <= kStatusSlot, "a slot per device state");
+struct StatusPage {
+  unsigned char *base;
+  uint64_t used;  // bit per slot
+};
+std::mutex g_status_mu;
+std::vector<StatusPage> g_status_pages;
+
+cudaError_t take_status_slot(DevState **out) {
+  std::lock_guard<std::mutex> lock(g_status_mu);
+  for (StatusPage &p : g_status_pages)
+    if (~p.used) {
+      const int i = __builtin_ctzll(~p.used);
+      p.used |= 1ull << i;
+      *out = (DevState *)(p.base + (size_t)i * kStatusSlot);
+      return cudaSuccess;
+    }
+  void *m = nullptr;
+  const cudaError_t e = cudaHostAlloc(&m, kStatusSlot * kStatusSlots, cudaHostAllocMapped | cudaHostAllocPortable);
+  if (e != cudaSuccess) return e;
+  g_status_pages.push_back({(unsigned char *)m, 1});
+  *out = (DevState *)m;
+  return cudaSuccess;
+}
+
+void give_status_slot(DevState *s) {
+  std::lock_guard<std::mutex> lock(g_status_mu);
+  size_t at = 0, empty = 0;
+  for (size_t k = 0; k < g_status_pages.size(); ++k) {
+    StatusPage &p = g_status_pages[k];
+    const size_t i = (size_t)((unsigned char *)s - p.base) / kStatusSlot;
+    if ((unsigned char *)s >= p.base && i < kStatusSlots) {
+      p.used &= ~(1ull << i);
+      at = k;
+    }
+    empty += p.used == 0;
+  }
+  if (empty < 2 || g_status_pages[at].used) return;
+  cudaFreeHost(g_status_pages[at].base);
+  g_status_pages.erase(g_status_pages.begin() + (long)at);
+}
+}  // namespace
+
 static void free_ctx(ll_ctx *c) {
   if (!c) return;
   int prev = 0;
@@ -1182,10 +1236,10 @@ static void free_ctx(ll_ctx *c) {
                   c->rowE, c->colF, c->rowW, c->rowWi, c->colW, c->colWi};
   for (void *p : ptrs)
     if (p) cudaFree(p);
-  if (c->host_st) cudaFreeHost(c->host_st);
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   if (c->graph) cudaGraphDestroy(c->graph);
   if (c->stream) cudaStreamDestroy(c->stream);
+  if (c->host_st) give_status_slot(c->host_st);  // (the cudaFree calls above waited for the device)
   cudaSetDevice(prev);
   delete c;
 }
@@ -1254,14 +1308,16 @@ static ll_status build_tables(ll_ctx *ctx) {
     if ((int)t.size() != ctx->shape.st->tw) return LL_ERR_SHAPE;
     CK(upload(&ctx->stwH, t));
   }
+  std::vector<double2> ptw;
   if (ctx->pipe_w) {
-    CK(upload(&ctx->ptwW, pipe_twiddles(W)));
+    ptw = pipe_twiddles(W);
+    CK(upload(&ctx->ptwW, ptw));
     std::vector<RowConst> rc(H);
     for (int m2 = 0; m2 < H; ++m2)
       rc[m2] = {rE[2 * m2], rE[2 * m2 + 1], rW[2 * m2], rW[2 * m2 + 1], rWi[2 * m2], rWi[2 * m2 + 1], 0.0};
     CK(upload(&ctx->rowC, rc));
   }
-  if (ctx->pipe_t) CK(upload(&ctx->ptwH, pipe_twiddles(H)));
+  if (ctx->pipe_t) CK(upload(&ctx->ptwH, ctx->pipe_w && W == H ? ptw : pipe_twiddles(H)));
   CK(upload(&ctx->rowE, rE));
   CK(upload(&ctx->rowW, rW));
   CK(upload(&ctx->rowWi, rWi));
@@ -1392,7 +1448,7 @@ ll_status ll_create(int device, uint32_t q, uint32_t n, const ll_tuning *tuning,
         (e = cudaMalloc((void **)&ctx->carry, carry_bytes)) != cudaSuccess ||
         (e = cudaMalloc((void **)&ctx->flags, flag_bytes)) != cudaSuccess ||
         (e = cudaMalloc((void **)&ctx->st, sizeof(DevState))) != cudaSuccess ||
-        (e = cudaHostAlloc((void **)&ctx->host_st, sizeof(DevState), cudaHostAllocMapped)) != cudaSuccess) {
+        (e = take_status_slot(&ctx->host_st)) != cudaSuccess) {
       rc = e == cudaErrorMemoryAllocation ? LL_ERR_NOMEM : cuda_fail(ctx, e, "cudaMalloc");
       break;
     }
@@ -1405,38 +1461,38 @@ ll_status ll_create(int device, uint32_t q, uint32_t n, const ll_tuning *tuning,
     if (ctx->pipe_w && (rc = encode_map(ctx)) != LL_OK) break;
     rc = build_tables(ctx);
     if (rc != LL_OK) break;
-    // The dynamic shared-memory limit is a per-function (not per-context)
-    // attribute: raise it to the largest size any context has needed.
+    // The dynamic shared-memory limits of this shape's kernels.  A specialised
+    // kernel has one size; the generic ones serve all shapes, and a limit belongs
+    // to the function, not to the context: it is raised to the largest size any
+    // context has needed.  (All kernels of the tables were set before, 250 calls.)
     {
+      const int sw = (int)shape_wide_smem(s), st = (int)shape_tall_smem(s);
+      auto limit = [&](const void *k, int bytes) {
+        if (k && e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+      };
       static std::mutex mu;
-      static size_t max_sw = 0, max_st = 0;
+      static int max_sw = 0, max_st = 0;
       std::lock_guard<std::mutex> lock(mu);
-      const size_t sw = std::max(max_sw, shape_wide_smem(s)), st = std::max(max_st, shape_tall_smem(s));
-      if ((e = cudaFuncSetAttribute(wide_kernel<EPT, WIDE_ITER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw)) != cudaSuccess ||
-          (e = cudaFuncSetAttribute(wide_kernel<EPT, WIDE_REPORT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw)) != cudaSuccess ||
-          (e = cudaFuncSetAttribute(wide_kernel<EPT, WIDE_INIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw)) != cudaSuccess ||
-          (e = cudaFuncSetAttribute(tall_kernel<EPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st)) != cudaSuccess) {
+      if (s.sw) {
+        for (const void *k : {(const void *)s.sw->iter, (const void *)s.sw->report, (const void *)s.sw->init, (const void *)s.sw->iter_batch})
+          limit(k, sw);
+      } else {
+        max_sw = std::max(max_sw, sw);
+        for (const void *k : {(const void *)wide_kernel<EPT, WIDE_ITER>, (const void *)wide_kernel<EPT, WIDE_REPORT>,
+                              (const void *)wide_kernel<EPT, WIDE_INIT>})
+          limit(k, max_sw);
+      }
+      if (s.st) {
+        limit((const void *)s.st->run, st);
+        limit((const void *)s.st->batch, st);
+      } else {
+        max_st = std::max(max_st, st);
+        limit((const void *)tall_kernel<EPT>, max_st);
+      }
+      if (e != cudaSuccess) {
         rc = cuda_fail(ctx, e, "cudaFuncSetAttribute");
         break;
       }
-      for (const auto &k : kWide)
-        if ((e = cudaFuncSetAttribute(k.iter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw)) != cudaSuccess ||
-            (e = cudaFuncSetAttribute(k.report, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw)) != cudaSuccess ||
-            (e = cudaFuncSetAttribute(k.init, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw)) != cudaSuccess ||
-            (e = cudaFuncSetAttribute(k.iter_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sw)) != cudaSuccess)
-          break;
-      for (const auto &k : kTall)
-        if (e == cudaSuccess &&
-            ((e = cudaFuncSetAttribute(k.run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st)) != cudaSuccess ||
-             (k.batch &&
-              (e = cudaFuncSetAttribute(k.batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st)) != cudaSuccess)))
-          break;
-      if (e != cudaSuccess) {
-        rc = cuda_fail(ctx, e, "cudaFuncSetAttribute (static)");
-        break;
-      }
-      max_sw = sw;
-      max_st = st;
     }
     // Programmatic dependent launch pays when a pass runs in a few waves (the
     // next pass's prologue overlaps this one's drain); with many waves it
