@@ -793,9 +793,21 @@ __device__ __forceinline__ void carry_join(double pk, double cin, double P0, dou
 // warp until its stores are visible.  Per iteration, against flags released
 // and acquired per warp: 128K 10.7 -> 10.0 us, 512K 14.7 -> 13.5, 18432K
 // 385 -> 366, 3200K 62.2 -> 61.6.
+//
+// Words beyond the exact range may carry any value.  Their fault is reported,
+// but the value must not look like an empty slot, or its taker would wait until
+// the limit: the high word of what is published stays below the empty one's
+// (which also makes a positive infinity or NaN a number; the fault stands).
 constexpr int kNoCarryByte = 0x7F, kNoCarryHi = 0x7F7F7F7F;
-__device__ __forceinline__ void put_carry(double *slot, double c) {
+__host__ __device__ constexpr int published_hi(int hi) { return hi < kNoCarryHi ? hi : kNoCarryHi - 1; }
+static_assert(published_hi(kNoCarryHi) != kNoCarryHi && published_hi(0x7FF00000) != kNoCarryHi &&
+                  published_hi(0x43400000) == 0x43400000 && published_hi((int)0xC3400000) == (int)0xC3400000,
+              "no carry looks like an empty slot, carries below 2^53 are left alone");
+__device__ __forceinline__ void set_slot(double *slot, double c) {
   asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(slot), "d"(c) : "memory");
+}
+__device__ __forceinline__ void put_carry(double *slot, double c) {
+  set_slot(slot, __hiloint2double(published_hi(__double2hiint(c)), __double2loint(c)));
 }
 __device__ __forceinline__ double peek_carry(const double *slot) {
   double c;
@@ -824,7 +836,7 @@ __device__ __forceinline__ void take_carries(double *c, AT at, DevState *st, lon
   }
   const double none = __hiloint2double(kNoCarryHi, kNoCarryHi);
 #pragma unroll
-  for (int r = 0; r < R; ++r) put_carry(at(r), none);
+  for (int r = 0; r < R; ++r) set_slot(at(r), none);
 }
 
 // floor(x / d) for x < 2^58 and d < 2^31: an FP64 estimate (off by at most
