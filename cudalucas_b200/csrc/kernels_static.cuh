@@ -731,9 +731,12 @@ struct WordSize {
 };
 __device__ __forceinline__ uint32_t turn_fraction(int e, double turn) { return (uint32_t)fma((double)e, turn, 0.5 * turn); }
 
-// The readings of a thread's words: the largest |t - rint(t)| in units of
-// 2^-32 (an FP64 sum puts it into the low word, one integer maximum of three
-// takes it from there) and the largest magnitudes of t by its high word
+// The readings of a thread's words: the largest |t - rint(t)| (below 1) by 32 of
+// its bits, without the sign and the top bit of the exponent, which is zero: 10
+// exponent and 22 fraction bits, so that one integer maximum of three takes a
+// pair of words.  Such a remainder is a few units in the last place of t and
+// fits.  (In units of 2^-32, as the low word of a sum with 2^20, small ones, of
+// words below 2^20, lost their last places.)  And the largest magnitudes of t by its high word
 // (positive ones as signed, negative ones as unsigned integers).  At 2^51 and
 // above (or NaN) a double has no fraction bits left for the roundoff reading,
 // and the exact carry split no longer holds.
@@ -741,8 +744,9 @@ struct Readings {
   uint32_t err = 0, neg = 0;
   int32_t pos = 0;
   __device__ __forceinline__ void words(double t0, double r0, double t1, double r1) {
-    err = __vimax3_u32(err, (uint32_t)__double2loint(__dadd_rn(fabs(t0 - r0), 0x1p20)),
-                       (uint32_t)__double2loint(__dadd_rn(fabs(t1 - r1), 0x1p20)));
+    const double d0 = t0 - r0, d1 = t1 - r1;
+    err = __vimax3_u32(err, __funnelshift_l(__double2loint(d0), __double2hiint(d0), 2),
+                       __funnelshift_l(__double2loint(d1), __double2hiint(d1), 2));
     pos = __vimax3_s32(pos, __double2hiint(t0), __double2hiint(t1));
     neg = __vimax3_u32(neg, (uint32_t)__double2hiint(t0), (uint32_t)__double2hiint(t1));
   }
@@ -754,7 +758,7 @@ struct Readings {
     const bool out = pos >= 0x43200000 || neg >= 0xC3200000u;
     const bool any = __any_sync(0xffffffffu, out);
     if ((threadIdx.x & 31) == 0) {
-      const uint32_t bits = __float_as_uint((float)e * 0x1p-32f);
+      const uint32_t bits = __float_as_uint((float)__hiloint2double((int)(e >> 2), (int)(e << 30)));
       if (bits > seen) atomicMax(&st->err_bits, bits);
       if (any) atomicOr(&st->fault, 2u);
     }
