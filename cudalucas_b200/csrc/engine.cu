@@ -1586,10 +1586,9 @@ ll_status ll_create(int device, uint32_t q, uint32_t n, const ll_tuning *tuning,
     ta.ph = ctx->ph; ta.W = s.W; ta.H = s.H; ta.N = ctx->N; ta.ts = ctx->ts; ta.tmask = (1 << ctx->ts) - 1; ta.q = q; ta.wait = kWaitCycles;
     WideArgs &wa = ctx->wa;
     if (ctx->pipe_w) {
-      // a multiple of the slots, about 32, of four units or more each
-      const int ns = ctx->pipe_w->slots, units = s.H / 2;
-      wa.chains = ns * std::max(1, std::min(32 / ns, units / (4 * ns)));
-      wa.chain_len = (units + wa.chains - 1) / wa.chains;
+      const RunOrder o = run_order(ctx->pipe_w->slots, s.H / 2);
+      wa.chains = o.chains;
+      wa.chain_len = o.len;
     }
     wa.ptw = ctx->ptwW; wa.rowC = ctx->rowC;
     wa.A = ctx->A; wa.stw = ctx->stwW; wa.xint = ctx->xint; wa.carry = ctx->carry; wa.flags = ctx->flags; wa.twW = ctx->twW;
@@ -2022,8 +2021,16 @@ int32_t ll_check_tables(void) {
     if ((int)stage_twiddles(k.rad, k.nrad).size() != k.extra) ++bad;
   for (const auto &k : kTall)
     if ((int)stage_twiddles(k.rad, k.nrad).size() != k.tw) ++bad;
-  for (const auto &k : kPipe)
+  int most = EPT * TMAX / 2;  // units of the longest columns
+  for (const auto &k : kTall) most = std::max(most, k.L / 2);
+  for (const auto &k : kPipe) {
     if ((int)pipe_twiddles(k.L).size() != k.tw) ++bad;
+    // rows of every even column length, a flag per run among the 64
+    for (int units = 1; k.wide && units <= most; ++units) {
+      const RunOrder o = run_order(k.slots, units);
+      if (o.chains > 64 || o.chains % k.slots || !run_order_ok(o)) ++bad;
+    }
+  }
   for (const auto &k : kCluster) {
     int L = 1, Lc = 1;
     for (int i = 0; i < k.nrad; ++i) L *= k.rad[i];

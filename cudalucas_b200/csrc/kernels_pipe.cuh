@@ -578,6 +578,52 @@ constexpr int wide_pipe_smem() {
 // an extra ticket at the start, which computes that predecessor as far as its
 // outgoing carries only (for unit 0 the last unit: the wrap, 2^q = 1); the
 // predecessor itself is not stored before the extra ticket has read it.
+struct RunOrder {
+  int units, chains, len;  // runs of `len` units (the last ones shorter, or empty)
+  // The unit of ticket k: run k % chains, its extra unit first; -1: none.
+  __host__ __device__ __forceinline__ int unit(int k) const {
+    const int i = k / chains, j = k - i * chains, first = j * len;
+    if (first >= units) return -1;
+    if (i == 0) return (j == 0 ? units : first) - 1;
+    return first + i - 1 < units ? first + i - 1 : -1;
+  }
+  __host__ __device__ __forceinline__ int tickets() const { return chains * (len + 1); }
+  __host__ __device__ __forceinline__ bool extra(int k) const { return k < chains; }
+  // whether u ends its run, and the run whose extra ticket then reads it
+  __host__ __device__ __forceinline__ bool tail(int u) const { return u % len == len - 1 || u == units - 1; }
+  __host__ __device__ __forceinline__ int reader(int u) const { return u == units - 1 ? 0 : u / len + 1; }
+};
+// A multiple of the slots, about 32 runs, of four units or more each.
+inline RunOrder run_order(int slots, int units) {
+  const int chains = slots * std::max(1, std::min(32 / slots, units / (4 * slots)));
+  return {units, chains, (units + chains - 1) / chains};
+}
+// What the pass relies on: every unit once; the unit before at an earlier ticket
+// (else CTAs could wait for one that has not been drawn), or, at the start of a
+// run, the run's extra ticket for it; that one before its unit is drawn, and
+// flagged by the unit that ends the run.
+inline bool run_order_ok(const RunOrder &o) {
+  std::vector<int> at((size_t)o.units, -1);
+  for (int k = o.chains; k < o.tickets(); ++k) {
+    const int u = o.unit(k);
+    if (u < 0) continue;
+    if (u >= o.units || at[(size_t)u] >= 0) return false;
+    at[(size_t)u] = k;
+  }
+  for (int u = 0; u < o.units; ++u) {
+    const int before = u == 0 ? o.units - 1 : u - 1;
+    if (at[(size_t)u] < 0) return false;
+    if (u % o.len == 0) {
+      const int k = u / o.len;
+      if (k >= o.chains || o.unit(k) != before || k >= at[(size_t)before] || !o.tail(before) || o.reader(before) != k)
+        return false;
+    } else if (at[(size_t)before] >= at[(size_t)u] || o.tail(before)) {
+      return false;
+    }
+  }
+  return true;
+}
+
 template <int M>
 __global__ void __launch_bounds__(Pipe<M>::NT, 1)
     wide_pipe(const __grid_constant__ TileMap map, const __grid_constant__ WideArgs a) {
@@ -618,21 +664,14 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1)
   __syncthreads();
   griddep_wait();
   griddep_release();
-  // ticket k: run k % chains, its extra unit first
-  const int chains = a.chains, len = a.chain_len;
-  auto unit = [&](int k) {
-    const int i = k / chains, j = k - i * chains, first = j * len;
-    if (first >= units) return -1;
-    if (i == 0) return (j == 0 ? units : first) - 1;
-    return first + i - 1 < units ? first + i - 1 : -1;
-  };
+  const RunOrder order{units, a.chains, a.chain_len};
   auto fill = [&](int k, int pos, int box, bool first) {
     const int slot = pos % NS;
     if (first) s_pos[slot] = pos;
-    const int u = k < chains * (len + 1) ? unit(k) : -1;
+    const int u = k < order.tickets() ? order.unit(k) : -1;
     if (u < 0) {
       if (first) {
-        unit_of[slot] = k < chains * (len + 1) ? -2 : -1;
+        unit_of[slot] = k < order.tickets() ? -2 : -1;
         slot_expect(&full[slot], 0);
       }
       return;
@@ -715,8 +754,8 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1)
       continue;
     }
     slot_full(&full[slot], parity);  // every thread sees the copies
-    const bool extra = k < chains;
-    const int u = unit(k);
+    const bool extra = order.extra(k);
+    const int u = order.unit(k);
     const RowCells cells{(uint32_t)(slot * P::SLOT + row * 16)};
     auto ord16 = [](int r) { return out_slot<16>(r); };
     double2 v[16];
@@ -760,7 +799,7 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1)
     // carries by shuffles, row 0 those of the unit before (unit 0 the last
     // unit's, shifted by one element).  The last unit of a run publishes
     // none: the run after it takes those of its extra ticket.
-    const bool tail = u % len == len - 1 || u == units - 1;  // of its run
+    const bool tail = order.tail(u);  // of its run
     if (row == 1 && (extra || !tail)) {
       double *out = gcd + (size_t)u * W + t;
 #pragma unroll
@@ -799,7 +838,7 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1)
 #pragma unroll
       for (int r = 0; r < 16; ++r) cell(smb, cells.base + (uint32_t)(t + r * TR) * 32) = x[slot16(r)];
     }
-    if (!extra && tail && idx == 0) await_extra(&a.flags[u == units - 1 ? 0 : u / len + 1], a.st, &s_dead, a.wait);
+    if (!extra && tail && idx == 0) await_extra(&a.flags[order.reader(u)], a.st, &s_dead, a.wait);
     done();
     if (!extra && lane == 0) {
       store_tile(&map, 4 * u, warp * 256, smb + slot * P::SLOT + warp * 8192);

@@ -162,7 +162,9 @@ int32_t ll_kernel_kinds(const ll_ctx *ctx);
  * specialised kernels whose stage-twiddle table (built on the host from the
  * recorded radix list) does not have the size the kernel reads, plus the
  * built-in launch preferences that do not give a specialised shape of their
- * width.  0 when consistent; needs no GPU. */
+ * width, plus the numbers of row units for which the order of the persistent
+ * row pass does not hold what the pass relies on.  0 when consistent; needs no
+ * GPU. */
 int32_t ll_check_tables(void);
 const char *ll_status_string(ll_status s);
 
