@@ -1025,16 +1025,15 @@ static double twiddle_bias(int M) {
 // [e*TR + c], then the stage-1 twiddles w_TR^(j0*v) at rows of odd stride.
 static std::vector<double2> pipe_twiddles(int L) {
   const int M = L / 256, TR = L / 16, SS = M | 1;
-  std::vector<double2> out((size_t)8 * TR + (M > 1 ? 16 * SS : 0), make_double2(0.0, 0.0));
+  std::vector<double2> out((size_t)8 * TR + 16 * SS, make_double2(0.0, 0.0));
   // sixteenths of a turn: entries 3, 6 and 7 (w8, w8, w16^3) a quarter back
   static const int power[8] = {8, 4, 2, 2, 1, 1, 1, 1}, root[8] = {0, 0, 0, 2 - 4, 0, 1, 2 - 4, 3 - 4};
   const long double bias = (long double)twiddle_bias(M) * 0x1p-53L;
   for (int c = 0; c < TR; ++c)
     for (int e = 0; e < 8; ++e)
       out[(size_t)e * TR + c] = cos_tan((unsigned long long)(L + power[e] * c + root[e] * (L / 16)), L, bias);
-  if (M > 1)
-    for (int j = 0; j < 16; ++j)
-      for (int v = 0; v < M; ++v) out[(size_t)8 * TR + j * SS + v] = unit_root((unsigned long long)j * v, TR);
+  for (int j = 0; j < 16; ++j)
+    for (int v = 0; v < M; ++v) out[(size_t)8 * TR + j * SS + v] = unit_root((unsigned long long)j * v, TR);
   return out;
 }
 

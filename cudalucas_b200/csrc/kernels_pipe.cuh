@@ -37,14 +37,15 @@
 
 template <int M>
 struct Pipe {
+  static_assert(M >= 4, "rows and columns of 1024 and more");
   static constexpr int L = 256 * M, TR = 16 * M, TU = 2 * TR;
   // groups: 16 warps of 128 registers per SM where whole groups allow it
-  static constexpr int NG = M == 1 ? 7 : M == 2 ? 7 : M == 3 ? 5 : M == 4 ? 4 : M == 5 ? 3 : M <= 8 ? 2 : 1;
+  static constexpr int NG = M == 4 ? 4 : M == 5 ? 3 : M <= 8 ? 2 : 1;
   static constexpr int NT = NG * TU;
   static constexpr int SLOT = 32 * L;                  // bytes of a unit
   static constexpr int SS = M | 1;                     // stride of the stage-1 twiddles (odd: bank spread)
   static constexpr int TW2 = 8 * TR, TW1 = 16 * SS;    // twiddle entries of stage 2 and stage 1
-  static constexpr int TWN = TW2 + (M > 1 ? TW1 : 0);
+  static constexpr int TWN = TW2 + TW1;
   // the slots that fit beside the row pass's tables (the column pass needs less)
   static constexpr int FIT = (227 * 1024 - 128 - (16 * TWN + 24 * TR + 64)) / (SLOT + 32 * 41 + 8);
   static constexpr int NS = FIT > 2 * NG ? 2 * NG : FIT;
@@ -134,13 +135,12 @@ __device__ __forceinline__ double2 root16(int e) {
   return q == 0 ? make_double2(x, y) : q == 1 ? make_double2(-y, x) : q == 2 ? make_double2(-x, -y) : make_double2(y, -x);
 }
 
-// Barriers of a group (named barrier id, TU threads; a warp for M = 1).
+// Barriers of a group (named barrier id, TU threads).
 template <int M>
 struct GroupSync {
   int id;
   __device__ __forceinline__ void operator()() const {
-    if constexpr (Pipe<M>::TU == 32) __syncwarp();
-    else asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(Pipe<M>::TU) : "memory");
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(Pipe<M>::TU) : "memory");
   }
 };
 // mbarriers of the slots: one arrival (the thread that issues the copies)
@@ -304,18 +304,11 @@ template <int M, int SIGN, class C, class SY, class SLOT0>
 __device__ __forceinline__ void pipe_first(unsigned char *sm, const C cells, const double2 *tw, int t, const C cells1,
                                            int it0, double2 *v, SLOT0 s0, SY sync) {
   constexpr int TR = 16 * M;
-  if constexpr (M > 1) {
 #pragma unroll
-    for (int r = 0; r < 16; ++r) cell(sm, cells.base + (uint32_t)(t + r * TR) * C::XB) = v[s0(r)];
-    sync();
-    pipe_stage1<M, SIGN, true>(sm, cells1, tw + Pipe<M>::TW2, it0);
-    sync();
-  } else {
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < 16; ++r) cell(sm, cells.base + (((uint32_t)t ^ cells.swz(r)) + r * 16) * C::XB) = v[s0(r)];
-    __syncwarp();
-  }
+  for (int r = 0; r < 16; ++r) cell(sm, cells.base + (uint32_t)(t + r * TR) * C::XB) = v[s0(r)];
+  sync();
+  pipe_stage1<M, SIGN, true>(sm, cells1, tw + Pipe<M>::TW2, it0);
+  sync();
   const uint32_t blk = cells.base + (uint32_t)((t >> 4) * 16 + (t & 15) * TR) * C::XB;
   const uint32_t x = cells.swz(t & 15);
 #pragma unroll
@@ -334,15 +327,10 @@ __device__ __forceinline__ void pipe_second(unsigned char *sm, const C cells, co
 #pragma unroll
   for (int i = 0; i < 16; ++i) cell(sm, blk + (((uint32_t)i ^ x) * C::XB)) = v[s0(i)];
   sync();
-  if constexpr (M > 1) {
-    pipe_stage1<M, SIGN, false>(sm, cells1, tw + Pipe<M>::TW2, it0);
-    sync();
+  pipe_stage1<M, SIGN, false>(sm, cells1, tw + Pipe<M>::TW2, it0);
+  sync();
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = cell(sm, cells.base + (uint32_t)(t + i * TR) * C::XB);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = cell(sm, cells.base + (((uint32_t)t ^ cells.swz(i)) + i * 16) * C::XB);
-  }
+  for (int i = 0; i < 16; ++i) v[i] = cell(sm, cells.base + (uint32_t)(t + i * TR) * C::XB);
   dft16_tw<SIGN>(v, [&](int e) { return tw[e * TR + t]; });
 }
 
