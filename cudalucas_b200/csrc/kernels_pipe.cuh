@@ -724,9 +724,9 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1)
     }
     // the next ticket of this slot, needed when the unit is done
     unsigned next = 0;
-    if (idx == 0) next = atomicAdd(&a.st->pipe_ticket, 1u);
+    if (idx == 0) next = *(volatile int *)&s_dead ? 0x7fffffffu : atomicAdd(&a.st->pipe_ticket, 1u);  // (no ticket: no fill)
     auto done = [&] {  // after a barrier since the last refill()
-      if (idx == 0) s_next[g] = *(volatile int *)&s_dead ? 0x7fffffff : (int)min(next, 0x7fffffffu);  // (no ticket: no fill)
+      if (idx == 0) s_next[g] = (int)min(next, 0x7fffffffu);
       fence_async_smem();
       if (idx == TU - 1) {
         const int np = pos + NG, ns = np % NS;
