@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(ClusterCfg<PR, TWR, PT, TC, C, RPC>::T, 1)
   const uint32_t next_cbar = mbar_remote(&s_cbar, (unsigned)(wrap ? 0 : rank + 1));
   uint32_t off = ta.st->offset;
   const uint32_t seen = ta.st->err_bits;
-  Readings rd;
+  Readings<> rd;
   double2 *rw = rows + row * RS;
 
   // tall-pass thread: column `col` (local slot) of pair pl, thread tc of TC

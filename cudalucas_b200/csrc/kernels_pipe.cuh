@@ -688,7 +688,7 @@ __global__ void __launch_bounds__(Pipe<M>::NT, 1)
     s_two[g][1] = two.s1;
   }
   const uint32_t seen = __ldcg(&a.st->err_bits);
-  Readings rd;
+  Readings<> rd;
   // refill of the group's last slot, each warp its box, once the stores that
   // the warp has issued have read it
   int refill_pos = -1;

@@ -738,17 +738,24 @@ __device__ __forceinline__ uint32_t turn_fraction(int e, double turn) { return (
 // units of 2^-32, as the low word of a sum with 2^20, small ones, of words below
 // 2^20, lost their last places; by 32 bits shifted out of both words the reading
 // cost 1 to 2 % of a pass: 1600K 37.5 / 37.7 us per iteration, 3200K 54.7, so 54.0,
-// 32768K 550 / 559, so 553.)  And the largest magnitudes of t by its high word
+// 32768K 550 / 559, so 553.)  Rows with few elements per thread take the magnitudes
+// instead (FEW: 32K 5.75 / 5.63, 50K 6.57 / 6.47; the others lose by it, 3200K 54.1 /
+// 54.4, 32768K 554 / 556).  And the largest magnitudes of t by its high word
 // (positive ones as signed, negative ones as unsigned integers).  At 2^51 and
 // above (or NaN) a double has no fraction bits left for the roundoff reading,
 // and the exact carry split no longer holds.
+template <bool FEW = false>
 struct Readings {
   uint32_t below = 0, neg = 0;
   int32_t above = 0, pos = 0;
   __device__ __forceinline__ void words(double t0, double r0, double t1, double r1) {
-    const int32_t d0 = __double2hiint(t0 - r0), d1 = __double2hiint(t1 - r1);
-    above = __vimax3_s32(above, d0, d1);
-    below = __vimax3_u32(below, (uint32_t)d0, (uint32_t)d1);
+    if constexpr (FEW) {
+      above = __vimax3_s32(above, __double2hiint(fabs(t0 - r0)), __double2hiint(fabs(t1 - r1)));
+    } else {
+      const int32_t d0 = __double2hiint(t0 - r0), d1 = __double2hiint(t1 - r1);
+      above = __vimax3_s32(above, d0, d1);
+      below = __vimax3_u32(below, (uint32_t)d0, (uint32_t)d1);
+    }
     pos = __vimax3_s32(pos, __double2hiint(t0), __double2hiint(t1));
     neg = __vimax3_u32(neg, (uint32_t)__double2hiint(t0), (uint32_t)__double2hiint(t1));
   }
@@ -965,7 +972,7 @@ __device__ __forceinline__ void wide_body(const WideArgs &a, int blk, S sync = S
     // (row, m1), the packed pair of carry_split and the outgoing carry.
     double2 *ks = sm + row * RS + t;  // ks[r*TR]: element m1 = t + r*TR
     double *gcd = reinterpret_cast<double *>(a.carry);
-    Readings rd;
+    Readings<> rd;
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
       const uint32_t D = a.colD[r];
@@ -1122,7 +1129,7 @@ __device__ __forceinline__ void wide_any_body(const WideArgs &a, int blk, S sync
     fall_stages<P, 0, 1, TR, -1, false, false>(stw, t, sync, ld_first, st_reg, ld, st);
     double2 *ks = rw + t;  // ks[r*TR]: element m1 = t + r*TR
     double *gcd = reinterpret_cast<double *>(a.carry);
-    Readings rd;
+    Readings<true> rd;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const uint32_t D = a.colD[r];
