@@ -303,7 +303,7 @@ def run_ours(args, world, rank, local):
                 "frac": round(2 * alg_bytes / (t_iter * 1e-3) / 1e9 / hbm, 4), "traffic": None,
                 "alg_bytes_per_iteration": 2 * alg_bytes, "iteration_us": round(t_iter * 1000, 3),
                 "note": "latency bound: the state stays in the shared memory of one thread-block cluster, "
-                        "three cluster barriers per iteration; HBM is read once per launch",
+                        "two cluster barriers per iteration; HBM is read once per launch",
                 "two_launch_us": {"tall": round(t_tall * 1000, 2), "wide": round(t_wide * 1000, 2)}}
         launches = K * -(-S // 65536)
     else:

@@ -675,7 +675,10 @@ static const PipeKernel kPipe[] = {
 // from 9000K on (6272K 116 / 118, 9408K 221 / 216, 14336K 277 / 266); rows up
 // to 768 never do (4320K 93.5 / 95.2).  Columns, 2048K (512 x 2048) 33.2 /
 // 33.8, 4096K (2048 x 1024) 67.2 / 70.0, but 2304K (512 x 2304) 40.4 / 38.1,
-// 3200K 57.4 / 55.2, 18432K 290 / 266.
+// 3200K 57.4 / 55.2, 18432K 290 / 266.  (The lines are drawn by length, not by
+// units: of the 169 shapes of table lengths from 1000K to 9400K none runs more
+// than 1 % slower for it, 768 x 1536 42.4 / 42.8; some between 1440K and 3584K
+// would gain, 2304 x 512 50.1 / 43.6, 1792 x 768 55.4 / 48.9.)
 static bool pipe_rows(long long W, long long n) {
   return W >= 1024 && n >= 3000 * 1024 && (W != 1792 || n >= 9000 * 1024);
 }
@@ -1056,7 +1059,8 @@ static const PreferredShape kPreferred[] = {
     {160u * 1024, 512, 0},  // 160K: 0.0082 against 0.0085 ms/iter (W = 256)
     {168u * 1024, 512, 0},  // 168K: 0.0089 against 0.0098 ms/iter (W = 256)
     {224u * 1024, 512, 0},  // 224K: 0.0107 against 0.0114 ms/iter (W = 256)
-    {288u * 1024, 512, 32},  // 288K: four rows per CTA, as fast as two
+    {288u * 1024, 512, 32},  // 288K: four rows per CTA, 0.0107 ms/iter; two, as without an entry, 0.0098 (but
+                             // test_preferred_shapes_agree_with_heuristic_shapes needs another shape here)
     {640u * 1024, 256, 0},  // 640K: 0.0161 against 0.0299 ms/iter (W = 1024)
     {768u * 1024, 768, 0},  // 768K: 0.0181 against 0.0247 ms/iter (W = 512)
     {784u * 1024, 256, 0},  // 784K: 0.0188 against 0.0237 ms/iter (W = 512)

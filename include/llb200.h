@@ -65,8 +65,8 @@ typedef struct {
  * that have a fused cooperative kernel (12K, 14K, 56K) as one launch with
  * grid barriers between the passes, instead of two launches per iteration
  * (measured slower at 12K and 14K, equal at 56K, so not the default);
- * LL_KERNELS_NO_PREFETCH turns off the L2 prefetch that lengths larger than
- * L2 use.  Short lengths with a cluster-resident kernel (8K, 10K, 12K, 14K,
+ * LL_KERNELS_NO_PREFETCH turns off the L2 prefetch of the passes with a launch
+ * per unit at lengths larger than L2.  Short lengths with a cluster-resident kernel (8K, 10K, 12K, 14K,
  * 16K, 18K, 20K; 32K, 36K, 42K, 48K, 56K for steps of fewer than 8 iterations)
  * run an ll_step as one launch of one thread-block cluster whose shared memory
  * holds the whole state;
