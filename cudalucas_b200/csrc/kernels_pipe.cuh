@@ -20,8 +20,8 @@
 // Measured (us per iteration, launch per unit -> persistent): 3200K 61.4 ->
 // 55.2, 8192K 141 -> 125, 18432K 366 -> 267, 32768K 796 -> 555; a row unit at
 // 18432K 39.5 K -> 25 K cycles, a column unit 24.0 K -> 19.8 K.  What bounds
-// them now is shared memory and the FP64 pipe in turn, 46 % and 44 % of the
-// time in the columns of 3072: its one group of twelve warps does both in step.
+// them now is shared memory and the FP64 pipe in turn, 58 % and 49 % of the
+// cycles in the columns of 3072: its one group of twelve warps does both in step.
 //
 // In-place order.  A transform takes elements t + r*TR (TR = 16*M, r < 16) in
 // thread t and leaves outputs c + r*TR in thread c:
